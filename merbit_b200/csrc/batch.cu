@@ -49,9 +49,10 @@ int pick_vw(int k, long long ldx, const void* x, const void* y, long long ldy, i
         if (vw == 1) return 1;
         const size_t a = (size_t)vw * esz;  // vector load size
         if (ldx % vw != 0) continue;
+        // the kernel keeps the distance of rows in 32 bits
+        if (std::max(ldx, ldy) > (long long)(UINT_MAX / (unsigned)esz)) continue;
         if (((uintptr_t)x % (a < 16 ? a : 16)) != 0) continue;
         (void)y;
-        (void)ldy;
         return vw;
     }
     return 1;
@@ -178,6 +179,12 @@ int batch_upload(merbit_batch_s* b, const std::vector<SpmmDesc>& h, long long to
         b->slots = SpmmSlots();
         int st = alloc_spmm_slots(&b->slots, tot * b->k, s);
         if (st != MERBIT_OK) return st;
+    } else {
+        // other tiles than before: every word empty again (a launch of the
+        // SpMM kernel empties only the words it uses)
+        MERBIT_CUDA(cudaDeviceSynchronize());  // launches may use them
+        MERBIT_CUDA(cudaMemsetAsync(b->slots.words, 0xFF,
+                                    sizeof(unsigned long long) * 4 * (size_t)b->slots.nslots, s));
     }
     MERBIT_CUDA(cudaStreamSynchronize(s));
     b->total_tiles = (int)tot;

@@ -10,19 +10,32 @@
 // (G groups per warp), lane j of a group owning RHS columns
 // [j*VW, j*VW + VW).  The x rows of the next CH nonzeros are gathered while
 // the current CH are accumulated, so gathers overlap the walk.  A row that
-// ends inside a segment is written directly (coalesced across the group's
-// lanes); the group segmented scan (shuffles with stride K/VW) finishes the
+// begins and ends inside a segment is written directly, as vectors where Y
+// allows it; the group segmented scan (shuffles with stride K/VW) finishes the
 // rows split between groups, and rows split between tiles are finished
-// per RHS column exactly as in the SpMV: two-tile rows by an atomicExch
+// per RHS column as in the SpMV: two-tile rows by an atomicExch
 // swap of the partials (the later side writes carry + head), longer rows by
-// a fixed-order look-back over published per-tile partials.  No float
-// atomics: results are bitwise reproducible.
+// a fixed-order look-back over the partials their tiles published, queued and
+// taken when the warp has no tile left.  No float atomics: results are bitwise
+// reproducible.
+//
+// What bounds it: instructions and the latency of the X-row gathers, not
+// bytes.  So the walk has no condition per nonzero: while no group of the warp
+// ends a row or its segment within a chunk (one vote), a chunk is loads and
+// arithmetic only; row ends take a branch of their own, a row's sum goes to Y
+// without passing through double when alpha = 1 and beta = 0, and only the
+// slots that a launch uses are emptied for the next one (all of them, they
+// were 20 MB of L2 for Zipf-1M at k = 16, whose X of 64 MB then no longer fit).
+// Measured on B200, before and after: Zipf-1M FP32 k = 16 526 -> 351 us, its
+// fused backward 628 -> 550; Zipf-500k FP64 k = 8 210 -> 153; 32 R-MAT
+// matrices FP32 in one launch, k = 4 603 -> 435, k = 32 1,540 -> 1,070.
 //
 // Batches: the tiles of all matrices form one index space; matrix m owns
 // tiles [tile_begin_m, tile_begin_m + num_tiles_m).  Warps of the
 // persistent cooperative grid take tiles round-robin, so one launch covers
 // the whole batch, and the launch can be captured in a CUDA graph and
-// replayed (carry slots are per launch parity, as in the SpMV).
+// replayed (carry slots come in two parities; a launch empties the words that
+// it uses in the other one, for the launch that follows).
 //
 // Fused backward (DV, merbit_spmm_dval): run on the transpose plan of A, the
 // walk also forms dL/dval for each nonzero from the G row it has just
@@ -76,6 +89,31 @@ __device__ __forceinline__ void st_row(Y* __restrict__ y, size_t off, double v, 
     y[off] = (Y)o;
 }
 
+// One lane's VW values of a Y row: a vector store where the address allows it
+// (vec), else one store per column.
+template <int VW>
+__device__ __forceinline__ void st_vec(float* p, const float (&o)[VW], bool vec) {
+    if (VW == 4 && vec) {
+        __stcs(reinterpret_cast<float4*>(p), make_float4(o[0], o[1 % VW], o[2 % VW], o[3 % VW]));
+    } else if (VW == 2 && vec) {
+        __stcs(reinterpret_cast<float2*>(p), make_float2(o[0], o[1 % VW]));
+    } else {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) p[v] = o[v];
+    }
+}
+template <int VW>
+__device__ __forceinline__ void st_vec(double* p, const double (&o)[VW], bool vec) {
+    if (VW >= 2 && vec) {
+#pragma unroll
+        for (int v = 0; v + 1 < VW; v += 2)
+            __stcs(reinterpret_cast<double2*>(p + v), make_double2(o[v], o[(v + 1) % VW]));
+    } else {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) p[v] = o[v];
+    }
+}
+
 __device__ __forceinline__ unsigned long long dbits(double v) {
     unsigned long long b = (unsigned long long)__double_as_longlong(v);
     return b == kEmpty ? 0x7FF8000000000000ull : b;
@@ -83,101 +121,214 @@ __device__ __forceinline__ unsigned long long dbits(double v) {
 
 }  // namespace
 
-// The VW accumulators of one lane.  Generic: one Acc per column.
-template <class Acc, int VW, typename P, typename X>
-struct AccRow {
-    static constexpr bool kPairs = false;
-    Acc a[VW];
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int v = 0; v < VW; ++v) a[v].zero();
-    }
-    __device__ __forceinline__ void add(P av, const X (&x)[VW]) {
-#pragma unroll
-        for (int v = 0; v < VW; ++v) a[v].add(av * (P)x[v]);
-    }
-    __device__ __forceinline__ double value(int v) const { return a[v].value(); }
-    __device__ __forceinline__ void add_pair(P a0, const X (&x0)[VW], P a1, const X (&x1)[VW]) {
-        add(a0, x0);
-        add(a1, x1);
-    }
-    // products formed beforehand (one per column)
-    __device__ __forceinline__ void add_p(const P (&p)[VW]) {
-#pragma unroll
-        for (int v = 0; v < VW; ++v) a[v].add(p[v]);
-    }
-};
-
-// TwoSum accumulators of an even number of columns, two columns per packed
-// f32x2 instruction (sm_100).  Every operation rounds as the scalar TwoSum of
-// AccTwoSum does (products rounded, then s + p with its exact error added
-// to c), so the results are bit-identical to the scalar form with half the
-// instructions.
-__device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
-    unsigned long long r;
+// Two floats in one 64-bit register pair, and arithmetic on both (sm_100).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 f2_pack(float lo, float hi) {
+    f32x2 r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
     return r;
 }
-__device__ __forceinline__ void f2_unpack(unsigned long long v, float& lo, float& hi) {
+__device__ __forceinline__ void f2_unpack(f32x2 v, float& lo, float& hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+    f32x2 r;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
+__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
+    f32x2 r;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
-                                                     unsigned long long c) {
-    unsigned long long r;
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
+    f32x2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+// r = a b + c where `on`; r stays where not
+__device__ __forceinline__ void f2_fma_if(bool on, f32x2& r, f32x2 a, f32x2 b, f32x2 c) {
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %4, 0;\n\t@p fma.rn.f32x2 %0, %1, %2, %3;\n\t}"
+        : "+l"(r)
+        : "l"(a), "l"(b), "l"(c), "r"((int)on));
+}
+
+// One lane's VW values of an X row, as they sit in registers: floats of an
+// even width in pairs (as the load delivers them and the packed arithmetic
+// takes them, so no moves), else one by one.
+template <typename X, int VW>
+struct XRow {
+    X r[VW];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) r[v] = (X)0;
+    }
+    __device__ __forceinline__ void load(const X* p) { ld_vec<VW>(p, r); }
+    __device__ __forceinline__ X operator[](int v) const { return r[v]; }
+};
+template <int VW>
+struct XPairs {
+    static_assert(VW == 2 || VW == 4, "pairs");
+    f32x2 r[VW / 2];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int h = 0; h < VW / 2; ++h) r[h] = 0ull;
+    }
+    __device__ __forceinline__ void load(const float* p) {
+        if constexpr (VW == 4) {
+            const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(p));
+            r[0] = t.x;
+            r[1] = t.y;
+        } else {
+            r[0] = __ldg(reinterpret_cast<const unsigned long long*>(p));
+        }
+    }
+    __device__ __forceinline__ float operator[](int v) const {
+        float lo, hi;
+        f2_unpack(r[v / 2], lo, hi);
+        return (v & 1) ? hi : lo;
+    }
+};
+template <>
+struct XRow<float, 2> : XPairs<2> {};
+template <>
+struct XRow<float, 4> : XPairs<4> {};
+
+// The VW accumulators of one lane.
+//   add, set     one product per column: into the sum, or as a row's first
+//   add_two      a0 x0 and, with `both`, a1 x1 of the same row
+//   add_p        products formed beforehand
+//   value        the sum in double; rounded: in the type of Y
+//   stash, unstash   to and from this lane's place in a shared-memory area
+//                    of 256 * VW bytes
+// F64: one double per column.
+template <class Acc, int VW, typename P, typename X>
+struct AccRow {
+    double a[VW];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) a[v] = 0.0;
+    }
+    __device__ __forceinline__ void add(P av, const XRow<X, VW>& x) {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) a[v] += av * (P)x[v];
+    }
+    __device__ __forceinline__ void set(P av, const XRow<X, VW>& x) {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) a[v] = 0.0 + av * (P)x[v];
+    }
+    __device__ __forceinline__ void add_two(P a0, const XRow<X, VW>& x0, P a1,
+                                            const XRow<X, VW>& x1, bool both = true) {
+        add(a0, x0);
+        if (both) add(a1, x1);
+    }
+    __device__ __forceinline__ void add_p(const P (&p)[VW]) {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) a[v] += p[v];
+    }
+    __device__ __forceinline__ double value(int v) const { return a[v]; }
+    __device__ __forceinline__ void rounded(X (&o)[VW]) const {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) o[v] = (X)a[v];
+    }
+    __device__ __forceinline__ void stash(unsigned char* p, int lane) const {
+        if constexpr (VW == 1) {
+            reinterpret_cast<double*>(p)[lane] = a[0];
+        } else {
+#pragma unroll
+            for (int h = 0; h < VW / 2; ++h)
+                reinterpret_cast<double2*>(p)[32 * h + lane] = make_double2(a[2 * h], a[2 * h + 1]);
+        }
+    }
+    __device__ __forceinline__ void unstash(const unsigned char* p, int lane) {
+        if constexpr (VW == 1) {
+            a[0] = reinterpret_cast<const double*>(p)[lane];
+        } else {
+#pragma unroll
+            for (int h = 0; h < VW / 2; ++h) {
+                const double2 t = reinterpret_cast<const double2*>(p)[32 * h + lane];
+                a[2 * h] = t.x;
+                a[2 * h + 1] = t.y;
+            }
+        }
+    }
+};
+
+// FP32/BF16, an even number of columns: TwoSum accumulators, two columns per
+// packed f32x2 instruction.  The steps are Knuth's, with n = s - t in the
+// place of -(t - s): t = s + q, e = (s - (t + n)) + (q + n).  A lone product
+// enters with its own rounding error (a x + n instead of q + n); two products
+// of one row enter as their fused sum, whose rounding is one unit of
+// |a0 x0| + |a1 x1|.
 template <int VW>
 struct AccRow<AccTwoSum, VW, float, float> {
     static_assert(VW % 2 == 0, "packed TwoSum needs an even width");
-    // two products of one row may enter as their fused sum: the pair's
-    // rounding (one unit of |a0 x0| + |a1 x1|) replaces the product's
-    static constexpr bool kPairs = true;
-    unsigned long long s[VW / 2], c[VW / 2];
+    using XR = XRow<float, VW>;
+    f32x2 s[VW / 2], c[VW / 2];
     __device__ __forceinline__ void zero() {
 #pragma unroll
         for (int h = 0; h < VW / 2; ++h) s[h] = c[h] = 0ull;  // +0.0f, +0.0f
     }
-    __device__ __forceinline__ void add(float av, const float (&x)[VW]) {
-        const unsigned long long a2 = f2_pack(av, av);
-#pragma unroll
-        for (int h = 0; h < VW / 2; ++h) sum(h, f2_mul(a2, f2_pack(x[2 * h], x[2 * h + 1])));
+    // t = s + q; (s, c) take t and its error, `qn` being q + n
+    __device__ __forceinline__ void finish(int h, f32x2 t, f32x2 n, f32x2 qn) {
+        c[h] = f2_add(c[h], f2_add(f2_sub(s[h], f2_add(t, n)), qn));
+        s[h] = t;
     }
-    __device__ __forceinline__ void add_pair(float a0, const float (&x0)[VW], float a1,
-                                             const float (&x1)[VW]) {
-        const unsigned long long b0 = f2_pack(a0, a0), b1 = f2_pack(a1, a1);
+    __device__ __forceinline__ void add(float av, const XR& x) {
+        const f32x2 a2 = f2_pack(av, av);
 #pragma unroll
         for (int h = 0; h < VW / 2; ++h) {
-            const unsigned long long p0 = f2_mul(b0, f2_pack(x0[2 * h], x0[2 * h + 1]));
-            sum(h, f2_fma(b1, f2_pack(x1[2 * h], x1[2 * h + 1]), p0));
+            const f32x2 t = f2_add(s[h], f2_mul(a2, x.r[h]));
+            const f32x2 n = f2_sub(s[h], t);
+            finish(h, t, n, f2_fma(a2, x.r[h], n));
+        }
+    }
+    __device__ __forceinline__ void set(float av, const XR& x) {
+        const f32x2 a2 = f2_pack(av, av);
+#pragma unroll
+        for (int h = 0; h < VW / 2; ++h) {
+            s[h] = f2_mul(a2, x.r[h]);
+            c[h] = f2_fma(a2, x.r[h], f2_sub(0ull, s[h]));
+        }
+    }
+    __device__ __forceinline__ void add_two(float a0, const XR& x0, float a1, const XR& x1) {
+        const f32x2 b0 = f2_pack(a0, a0), b1 = f2_pack(a1, a1);
+#pragma unroll
+        for (int h = 0; h < VW / 2; ++h) {
+            const f32x2 q = f2_fma(b1, x1.r[h], f2_mul(b0, x0.r[h]));
+            const f32x2 t = f2_add(s[h], q);
+            const f32x2 n = f2_sub(s[h], t);
+            finish(h, t, n, f2_add(q, n));
+        }
+    }
+    // the same when only some lanes of the warp have a second product
+    __device__ __forceinline__ void add_two(float a0, const XR& x0, float a1, const XR& x1,
+                                            bool both) {
+        const f32x2 b0 = f2_pack(a0, a0), b1 = f2_pack(a1, a1);
+#pragma unroll
+        for (int h = 0; h < VW / 2; ++h) {
+            f32x2 q = f2_mul(b0, x0.r[h]);
+            f2_fma_if(both, q, b1, x1.r[h], q);
+            const f32x2 t = f2_add(s[h], q);
+            const f32x2 n = f2_sub(s[h], t);
+            f32x2 qn = f2_add(q, n);
+            f2_fma_if(!both, qn, b0, x0.r[h], n);
+            finish(h, t, n, qn);
         }
     }
     __device__ __forceinline__ void add_p(const float (&p)[VW]) {
 #pragma unroll
-        for (int h = 0; h < VW / 2; ++h) sum(h, f2_pack(p[2 * h], p[2 * h + 1]));
-    }
-    // TwoSum of p into (s[h], c[h])
-    __device__ __forceinline__ void sum(int h, unsigned long long p) {
-        const unsigned long long t = f2_add(s[h], p);
-        const unsigned long long bp = f2_sub(t, s[h]);
-        const unsigned long long e = f2_add(f2_sub(s[h], f2_sub(t, bp)), f2_sub(p, bp));
-        s[h] = t;
-        c[h] = f2_add(c[h], e);
+        for (int h = 0; h < VW / 2; ++h) {
+            const f32x2 q = f2_pack(p[2 * h], p[2 * h + 1]);
+            const f32x2 t = f2_add(s[h], q);
+            const f32x2 n = f2_sub(s[h], t);
+            finish(h, t, n, f2_add(q, n));
+        }
     }
     __device__ __forceinline__ double value(int v) const {
         float s0, s1, c0, c1;
@@ -185,21 +336,123 @@ struct AccRow<AccTwoSum, VW, float, float> {
         f2_unpack(c[v / 2], c0, c1);
         return (v & 1) ? (double)s1 + (double)c1 : (double)s0 + (double)c0;
     }
+    __device__ __forceinline__ void rounded(float (&o)[VW]) const {
+#pragma unroll
+        for (int h = 0; h < VW / 2; ++h) f2_unpack(f2_add(s[h], c[h]), o[2 * h], o[2 * h + 1]);
+    }
+    __device__ __forceinline__ void stash(unsigned char* p, int lane) const {
+#pragma unroll
+        for (int h = 0; h < VW / 2; ++h)
+            reinterpret_cast<ulonglong2*>(p)[32 * h + lane] = make_ulonglong2(s[h], c[h]);
+    }
+    __device__ __forceinline__ void unstash(const unsigned char* p, int lane) {
+#pragma unroll
+        for (int h = 0; h < VW / 2; ++h) {
+            const ulonglong2 t = reinterpret_cast<const ulonglong2*>(p)[32 * h + lane];
+            s[h] = t.x;
+            c[h] = t.y;
+        }
+    }
 };
+// FP32/BF16, one column.
 template <>
 struct AccRow<AccTwoSum, 1, float, float> {
-    static constexpr bool kPairs = false;
+    using XR = XRow<float, 1>;
     AccTwoSum a;
     __device__ __forceinline__ void zero() { a.zero(); }
-    __device__ __forceinline__ void add(float av, const float (&x)[1]) { a.add(av * x[0]); }
-    __device__ __forceinline__ double value(int) const { return a.value(); }
-    __device__ __forceinline__ void add_pair(float a0, const float (&x0)[1], float a1,
-                                             const float (&x1)[1]) {
+    __device__ __forceinline__ void add(float av, const XR& x) { a.add(av * x[0]); }
+    __device__ __forceinline__ void set(float av, const XR& x) {
+        a.zero();
+        add(av, x);
+    }
+    __device__ __forceinline__ void add_two(float a0, const XR& x0, float a1, const XR& x1,
+                                            bool both = true) {
         add(a0, x0);
-        add(a1, x1);
+        if (both) add(a1, x1);
     }
     __device__ __forceinline__ void add_p(const float (&p)[1]) { a.add(p[0]); }
+    __device__ __forceinline__ double value(int) const { return a.value(); }
+    __device__ __forceinline__ void rounded(float (&o)[1]) const { o[0] = __fadd_rn(a.s, a.c); }
+    __device__ __forceinline__ void stash(unsigned char* p, int lane) const {
+        reinterpret_cast<float2*>(p)[lane] = make_float2(a.s, a.c);
+    }
+    __device__ __forceinline__ void unstash(const unsigned char* p, int lane) {
+        const float2 t = reinterpret_cast<const float2*>(p)[lane];
+        a.s = t.x;
+        a.c = t.y;
+    }
 };
+
+// A row that began two or more tiles before the tile that completes it: its
+// carry-in is the sum of the partials of the tiles in between, which other
+// warps process at about the same time.  The completing tile leaves its own
+// part (the head) in its boundary-swap slot, which such a row does not use,
+// and queues the look-back; the warp takes it when the queue is full, else
+// after its last tile, so that it does not wait for tiles while it has others
+// to process.  (Taken on the spot, the look-backs held up Zipf-1M at k = 16
+// for a third of its time.)
+struct SpmmLookBack {
+    void* y;    // the row of Y
+    int head;   // the completing tile (its slots hold the head)
+    int first;  // the tile in which the row begins
+};
+constexpr int kSpmmLookBacks = 8;
+
+// One look-back by one warp: lane l takes column l % K of tiles first + l / K,
+// + 32 / K, ...; R loads are in flight before any is summed, so a row of
+// hundreds of tiles takes few round trips.  The order of the sums depends only
+// on the tiles.
+template <int K, typename Y>
+__device__ __forceinline__ void spmm_look_back(const SpmmLookBack& e, unsigned long long* slots,
+                                               unsigned long long* xch, LaunchState* st,
+                                               double alpha, double beta, int lane) {
+    constexpr int TPS = 32 / K;
+    constexpr int R = 8;
+    const int j = lane % K;
+    double sum = 0.0;
+    for (int t = e.first + lane / K; t < e.head; t += TPS * R) {
+        unsigned long long bits[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            bits[r] = t + r * TPS < e.head ? ld_relaxed_u64(slots + (size_t)(t + r * TPS) * K + j) : 0ull;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (bits[r] == kEmpty) {  // not published yet: wait (bounded)
+                const unsigned long long* p = slots + (size_t)(t + r * TPS) * K + j;
+                const unsigned long long t0 = global_timer_ns();
+                while ((bits[r] = ld_relaxed_u64(p)) == kEmpty) {
+                    __nanosleep(32);
+                    if (*(volatile int*)&st->error != 0) break;
+                    if (global_timer_ns() - t0 > kCarryWaitNs) {
+                        atomicExch(&st->error, (int)MERBIT_ERR_TIMEOUT);
+                        break;
+                    }
+                }
+                if (bits[r] == kEmpty) bits[r] = 0ull;
+            }
+            sum += __longlong_as_double((long long)bits[r]);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = K; o < 32; o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    if (lane < K) {
+        const double head =
+            __longlong_as_double((long long)ld_relaxed_u64(xch + (size_t)e.head * K + j));
+        st_row(static_cast<Y*>(e.y), j, sum + head, alpha, beta);
+    }
+}
+
+template <int K, typename Y>
+__device__ __forceinline__ void drain_spmm_look_backs(const SpmmLookBack* q, int n,
+                                                      const SpmmLaunch& a, unsigned epoch,
+                                                      int lane) {
+    __syncwarp();
+    const size_t par = (size_t)(epoch & 1u) * a.nslots;
+    for (int i = 0; i < n; ++i)
+        spmm_look_back<K, Y>(q[i], a.slots + par, a.xch + par, a.state, a.alpha, a.beta, lane);
+    __syncwarp();
+}
 
 // DV: also form dL/dval for each nonzero (SpmmLaunch::dv_*), from the x row
 // the walk gathers anyway and the current row of dv_x.
@@ -227,7 +480,8 @@ struct SpmmTile {
     static constexpr bool STAGEP = K == 2 && VW == 2 && (ITEMS == 224 || ITEMS == 352) && !DV;
     static constexpr int NJ = ITEMS / 32;  // staged products per lane
     static constexpr int CAP = ITEMS + 32;
-    static constexpr int RPC = ITEMS + 16;  // row_ptr window (any rows per tile)
+    static constexpr int RPC = ITEMS + 16;  // row_ptr window (any rows per tile, and the
+                                            // end of the row that goes on after it)
     static constexpr size_t rp_bytes = a16((size_t)RPC * 4);
     static constexpr size_t col_bytes = a16((size_t)CAP * 4);
     static constexpr size_t val_bytes = a16((size_t)CAP * sizeof(V));
@@ -236,7 +490,10 @@ struct SpmmTile {
     static constexpr size_t perm_offset = rp_bytes + col_bytes + val_bytes;
     static constexpr size_t prod_bytes = STAGEP ? a16((size_t)ITEMS * VW * sizeof(P)) : 0;
     static constexpr size_t prod_offset = perm_offset + perm_bytes;
-    static constexpr size_t bar_offset = prod_offset + prod_bytes;
+    // each lane's first finished row of its segment, kept until the scan
+    static constexpr size_t first_offset = prod_offset + prod_bytes;
+    static constexpr size_t first_bytes = (size_t)256 * VW;
+    static constexpr size_t bar_offset = first_offset + first_bytes;
     static constexpr size_t bytes = bar_offset + 16;
     static constexpr int GV = 16 / (int)sizeof(V);
     static_assert(LPG >= 1 && LPG <= 32 && 32 % LPG == 0, "K/VW must divide 32");
@@ -252,6 +509,7 @@ struct SpmmTile {
         V* s_val = reinterpret_cast<V*>(ws + rp_bytes + col_bytes);
         const V* vals = static_cast<const V*>(d.vals);
         const int nrp = d.nrow + 1;
+        const int rp_end = min(c1.y + 2, nrp);  // the trailing row's end too
         // bulk copies need 16-byte aligned global addresses; an array whose
         // base is not 16-byte aligned (a caller's offset view) is staged by
         // plain loads instead (no transaction bytes)
@@ -261,7 +519,7 @@ struct SpmmTile {
             const int b_end = min((e + g - 1) & ~(g - 1), lim);
             return b_end > base ? (unsigned)(b_end - base) * (unsigned)esz : 0u;
         };
-        const unsigned tot = bb(d.row_ptr, c0.y, c1.y + 1, nrp, 4, 4) +
+        const unsigned tot = bb(d.row_ptr, c0.y, rp_end, nrp, 4, 4) +
                              bb(d.col, c0.x, c1.x, d.nnz, 4, 4) +
                              bb(vals, c0.x, c1.x, d.nnz, GV, (int)sizeof(V)) +
                              (DV ? bb(perm, c0.x, c1.x, d.nnz, 4, 4) : 0u);
@@ -286,24 +544,19 @@ struct SpmmTile {
             const int p0 = max(b_end, s);
             if (lane < e - p0) dst[p0 + lane - base] = src[p0 + lane];
         };
-        stage(s_rp, d.row_ptr, c0.y, c1.y + 1, nrp);
+        stage(s_rp, d.row_ptr, c0.y, rp_end, nrp);
         stage(s_col, d.col, c0.x, c1.x, d.nnz);
         stage(s_val, vals, c0.x, c1.x, d.nnz);
         if (DV) stage(reinterpret_cast<int*>(ws + perm_offset), perm, c0.x, c1.x, d.nnz);
     }
 
-    // Row ends of the tile as nonzero positions relative to x0.
-    static __device__ __forceinline__ int row_end(const int* s_rp, int rpo, int r, int x0) {
-        return s_rp[rpo + r + 1] - x0;
-    }
-
     static __device__ __forceinline__ void process(const SpmmLaunch& a, const SpmmDesc& d,
                                                    int u, int lt, unsigned epoch,
-                                                   unsigned char* ws, int lane) {
+                                                   unsigned char* ws, int lane,
+                                                   SpmmLookBack* lbq, int& nlb) {
         unsigned long long* slots = a.slots;
         unsigned long long* xch = a.xch;
         const int nslots = a.nslots;
-        LaunchState* st = a.state;
         const int* s_rp = reinterpret_cast<const int*>(ws);
         const int* s_col = reinterpret_cast<const int*>(ws + rp_bytes);
         const V* s_val = reinterpret_cast<const V*>(ws + rp_bytes + col_bytes);
@@ -313,153 +566,265 @@ struct SpmmTile {
         const int x0 = c0.x, y0 = c0.y, x1 = c1.x, y1 = c1.y;
         const int nz = x1 - x0, nr = y1 - y0, L = nz + nr;
         const int rpo = y0 - (y0 & ~3);
-        const int col_o = x0 - (x0 & ~3);
-        const int val_o = x0 - (x0 & ~(GV - 1));
         const int g = lane / LPG;        // group
         const int jl = lane % LPG;       // lane within group
         const int j0 = jl * VW;          // first RHS column of this lane
-        const X* __restrict__ xm = static_cast<const X*>(d.x);
-        Y* __restrict__ ym = static_cast<Y*>(d.y);
+        // this lane's columns of X, and the distance of its rows in bytes (32
+        // bits with vector loads: one wide multiply-add per address)
+        using Step = typename std::conditional<(VW > 1), unsigned, unsigned long long>::type;
+        const char* __restrict__ xl =
+            reinterpret_cast<const char*>(static_cast<const X*>(d.x) + j0);
+        const Step xstep = (Step)((unsigned long long)d.ldx * sizeof(X));
+        char* __restrict__ yl = reinterpret_cast<char*>(static_cast<Y*>(d.y) + j0);
+        const Step ystep = (Step)((unsigned long long)d.ldy * sizeof(Y));
+        auto y_row = [&](int r) {  // row r of the matrix
+            return reinterpret_cast<Y*>(yl + (unsigned long long)(unsigned)r * ystep);
+        };
+        const int nrow = d.nrow;
         const double alpha = a.alpha, beta = a.beta;
+        // plain product: a row's sum is rounded to Y as it is
+        const bool plain = alpha == 1.0 && beta == 0.0;
+        // Y rows of this lane start on its vector width
+        const bool vecy = VW > 1 && (((uintptr_t)yl | ystep) &
+                                     (VW * sizeof(Y) < 16 ? VW * sizeof(Y) - 1 : 15)) == 0;
+        // row r of Y from its sum in double
+        auto finish_row = [&](int r, const double (&v)[VW]) {
+            Y* yr = y_row(r);
+            if (plain) {
+                Y o[VW];
+#pragma unroll
+                for (int q = 0; q < VW; ++q) o[q] = (Y)v[q];
+                st_vec<VW>(yr, o, vecy);
+            } else {
+#pragma unroll
+                for (int q = 0; q < VW; ++q) st_row(yr, q, v[q], alpha, beta);
+            }
+        };
 
-        // ---- this group's segment [ds, de) of the tile's merge path
-        const int ds = min(g * SEG, L), de = min(ds + SEG, L);
-        auto search = [&](int dl, int& lx, int& ly) {
-            int lo = max(dl - nz, 0), hi = min(dl, nr);
+        // ---- this group's segment of the tile's merge path; it ends where
+        // the next group's starts.  Nonzeros are counted as in the whole
+        // matrix: rp_t[r] is the end of the tile's row r - 1, col_t[e] and
+        // val_t[e] belong to nonzero e.
+        const int* rp_t = s_rp + rpo;
+        const int* col_t = s_col - (x0 & ~3);
+        const V* val_t = s_val - (x0 & ~(GV - 1));
+        int lx, ly;
+        {
+            const int ds = min(g * SEG, L);
+            int lo = max(ds - nz, 0), hi = min(ds, nr);
             while (lo < hi) {
                 const int mid = (lo + hi) >> 1;
-                if (s_rp[rpo + mid + 1] - x0 <= dl - mid - 1)
+                if (rp_t[mid + 1] - x0 <= ds - mid - 1)
                     lo = mid + 1;
                 else
                     hi = mid;
             }
             ly = lo;
-            lx = dl - lo;
-        };
-        int lx, ly, lx_end, ly_end;
-        search(ds, lx, ly);
-        search(de, lx_end, ly_end);
+            lx = x0 + ds - lo;
+        }
+        int lx_end = x1, ly_end = nr;
+        if (G > 1) {
+            const int tx = __shfl_down_sync(0xFFFFFFFFu, lx, LPG);
+            const int ty = __shfl_down_sync(0xFFFFFFFFu, ly, LPG);
+            if (g < G - 1) {
+                lx_end = tx;
+                ly_end = ty;
+            }
+        }
 
         AccRow<Acc, VW, P, X> acc;
         acc.zero();
-        constexpr bool AccPairs = AccRow<Acc, VW, P, X>::kPairs;
-        int first_row = -1;
-        double first_val[VW];
+        unsigned char* s_first = ws + first_offset;
+        const bool any_end = ly < ly_end;  // a row ends in this segment
+        // The row open where the segment starts (`open`: it began before, in an
+        // earlier group or tile) is kept for the scan when it ends here; the
+        // rows that begin and end in the segment go to Y.  Rows without
+        // nonzeros are written after the walk.
+        const int first_row = ly;
+        bool open = any_end && rp_t[ly] < lx;
+        const bool had_open = open;
+        // end of the current row (INT_MAX past the segment's last row), kept in
+        // a register so the walk reads row_ptr once per row, not per nonzero;
+        // lim: the nonzero at which the current row or the segment ends
+        int next_end, lim;
+        auto next_row = [&](int e) {  // the first row from ly on that ends beyond e
+            for (;;) {
+                next_end = ly < ly_end ? rp_t[ly + 1] : INT_MAX;
+                if (next_end > e) break;
+                ++ly;
+            }
+            lim = min(next_end, lx_end);
+        };
+        if (open && rp_t[ly + 1] == lx) {  // its nonzeros all came before
+            acc.stash(s_first, lane);
+            open = false;
+            ++ly;
+        }
+        next_row(lx);
+
+        // fused dval: this lane's VW values of dv_x's current row, and of the
+        // row after it (loaded one row ahead: a row start would otherwise
+        // wait for its load)
+        const int* perm_t = reinterpret_cast<const int*>(ws + perm_offset) - (x0 & ~3);
+        XRow<X, VW> xrow, xnext;
+        int xnext_of = 0;
+        auto dv_load = [&](int r, XRow<X, VW>& o) {
+            if (r <= ly_end && y0 + r < nrow)
+                o.load(static_cast<const X*>(a.dv_x) + (size_t)(y0 + r) * a.dv_ldx + j0);
+        };
+        auto dv_next = [&]() {  // ly is the current row
+            if (xnext_of == ly)
+                xrow = xnext;
+            else
+                dv_load(ly, xrow);
+            xnext_of = ly + 1;
+            dv_load(xnext_of, xnext);
+        };
+        if (DV) {
+            xrow.zero();
+            xnext.zero();
+            xnext_of = -1;
+            dv_next();
+        }
+        const unsigned gmask = LPG == 32 ? 0xFFFFFFFFu : (((1u << LPG) - 1u) << (g * LPG));
+        // dval of nonzero e (and e + 1 of the same row): in the x type, VW
+        // fused multiply-adds per lane, then a tree over the group's lanes
+        // (error within (VW + log2 LPG) roundings of sum |g x|)
+        auto dv_dot = [&](const XRow<X, VW>& xr) {
+            X dd = (X)0;
 #pragma unroll
-        for (int v = 0; v < VW; ++v) first_val[v] = 0.0;
-        auto emit = [&](int r) {
-            if (first_row < 0) {
-                first_row = r;
+            for (int v = 0; v < VW; ++v) dd = fma(xr[v], xrow[v], dd);
+            return dd;
+        };
+        X* __restrict__ dvo = static_cast<X*>(a.dv_out);
+        auto dv_one = [&](int e, const XRow<X, VW>& xr) {
+            X dd = dv_dot(xr);
 #pragma unroll
-                for (int v = 0; v < VW; ++v) first_val[v] = acc.value(v);
+            for (int o = 1; o < LPG; o <<= 1) dd += __shfl_xor_sync(gmask, dd, o);
+            if (jl == 0) dvo[perm_t[e]] = dd;
+        };
+        auto dv_two = [&](int e, const XRow<X, VW>& xr0, const XRow<X, VW>& xr1) {
+            const X d0 = dv_dot(xr0), d1 = dv_dot(xr1);
+            if (LPG == 1) {
+                dvo[perm_t[e]] = d0;
+                dvo[perm_t[e + 1]] = d1;
             } else {
+                // even lanes sum the first, odd lanes the second: one exchange
+                // halves the two trees into one
+                const bool odd = (jl & 1) != 0;
+                X dd = (odd ? d1 : d0) + __shfl_xor_sync(gmask, odd ? d0 : d1, 1);
 #pragma unroll
-                for (int v = 0; v < VW; ++v)
-                    st_row(ym, (size_t)(y0 + r) * d.ldy + j0 + v, acc.value(v), alpha, beta);
+                for (int o = 2; o < LPG; o <<= 1) dd += __shfl_xor_sync(gmask, dd, o);
+                if (jl < 2) dvo[perm_t[e + jl]] = dd;
+            }
+        };
+
+        // the current row ends at nonzero e
+        auto end_row = [&](int e) {
+            if (open) {
+                acc.stash(s_first, lane);
+                open = false;
+            } else if (plain) {
+                Y o[VW];
+                acc.rounded(o);
+                st_vec<VW>(y_row(y0 + ly), o, vecy);
+            } else {
+                Y* yr = y_row(y0 + ly);
+#pragma unroll
+                for (int v = 0; v < VW; ++v) st_row(yr, v, acc.value(v), alpha, beta);
             }
             acc.zero();
+            ++ly;
+            next_row(e);
+            if (DV) dv_next();
         };
 
         // ---- walk: chunks of CH nonzeros, the next chunk's x rows in flight
         // (two named buffers, so both stay in registers)
-        X xa[CH][VW], xb[CH][VW];
+        XRow<X, VW> xa[CH], xb[CH];
         V va[CH], vb[CH];
-        auto load_chunk = [&](int c, X (&xr)[CH][VW], V (&vv)[CH]) {
+        // (past the segment's end a nonzero of the tile is read again: loads
+        // without conditions; used only when the tile has nonzeros)
+        const int e_last = max(lx_end - 1, x0);
+        auto load_chunk = [&](int c, XRow<X, VW> (&xr)[CH], V (&vv)[CH]) {
 #pragma unroll
             for (int t = 0; t < CH; ++t) {
-                if (c + t < lx_end) {
-                    const int e = c + t;
-                    const int colv = s_col[col_o + e];
-                    vv[t] = s_val[val_o + e];
-                    ld_vec<VW>(xm + (size_t)colv * d.ldx + j0, xr[t]);
-                }
+                const int e = min(c + t, e_last);
+                const unsigned colv = (unsigned)col_t[e];
+                vv[t] = val_t[e];
+                xr[t].load(reinterpret_cast<const X*>(xl + (unsigned long long)colv * xstep));
             }
         };
-        // end of row ly (INT_MAX past the segment's last row), kept in a
-        // register so the walk reads row_ptr once per row, not per nonzero
-        int next_end = ly < ly_end ? row_end(s_rp, rpo, ly, x0) : INT_MAX;
-        // fused dval: this lane's VW values of dv_x's current row
-        const X* __restrict__ dvx = static_cast<const X*>(a.dv_x);
-        X* __restrict__ dvo = static_cast<X*>(a.dv_out);
-        X xrow[VW];
-        int xrow_of = -1;
-        const int* s_perm = reinterpret_cast<const int*>(ws + perm_offset);
-        const unsigned gmask = LPG == 32 ? 0xFFFFFFFFu : (((1u << LPG) - 1u) << (g * LPG));
-        auto dv_step = [&](int t, int e, const X (&xr)[CH][VW]) {
-            if (y0 + ly != xrow_of) {  // uniform within the group
-                xrow_of = y0 + ly;
-                ld_vec<VW>(dvx + (size_t)xrow_of * a.dv_ldx + j0, xrow);
-            }
-            // in the x type: VW fused multiply-adds per lane, then a tree
-            // over the group's lanes (error within (VW + log2 LPG) roundings
-            // of sum |g x|)
-            X dd = (X)0;
+        // nonzeros c .. c + CH - 1 (those below lx_end); every row that ends at
+        // or before c is finished, so c belongs to row ly.  Called by all
+        // lanes of the warp.
+        auto consume = [&](int c, const XRow<X, VW> (&xr)[CH], const V (&vv)[CH]) {
+            if (__all_sync(0xFFFFFFFFu, lim > c + CH)) {  // no row or segment ends here
+                if constexpr (CH == 2) {
+                    // F32/BF16: one compensated addition of the fused pair
+                    acc.add_two(to_p(vv[0]), xr[0], to_p(vv[1]), xr[1]);
+                    if (DV) dv_two(c, xr[0], xr[1]);
+                } else {
 #pragma unroll
-            for (int v = 0; v < VW; ++v) dd = fma(xr[t][v], xrow[v], dd);
-#pragma unroll
-            for (int o = LPG / 2; o > 0; o >>= 1) dd += __shfl_xor_sync(gmask, dd, o);
-            if (jl == 0) dvo[s_perm[col_o + e]] = dd;
-        };
-        auto end_rows = [&](int e) {
-            while (next_end <= e) {
-                emit(ly);
-                ++ly;
-                next_end = ly < ly_end ? row_end(s_rp, rpo, ly, x0) : INT_MAX;
-            }
-        };
-        auto consume = [&](int c, const X (&xr)[CH][VW], const V (&vv)[CH]) {
-            if (AccPairs && CH == 2) {
-                // two nonzeros of one row: one compensated addition of their
-                // fused pair sum (fma(a1, x1, a0 x0)) instead of two
-                if (c < lx_end) {
-                    end_rows(c);
-                    if (c + 1 < lx_end && next_end > c + 1) {
-                        acc.add_pair(to_p(vv[0]), xr[0], to_p(vv[1]), xr[1 % CH]);
-                        if (DV) {
-                            dv_step(0, c, xr);
-                            dv_step(1 % CH, c + 1, xr);
-                        }
-                        return;
-                    }
-                    acc.add(to_p(vv[0]), xr[0]);
-                    if (DV) dv_step(0, c, xr);
-                    if (c + 1 < lx_end) {
-                        end_rows(c + 1);
-                        acc.add(to_p(vv[1 % CH]), xr[1 % CH]);
-                        if (DV) dv_step(1 % CH, c + 1, xr);
+                    for (int t = 0; t < CH; ++t) {
+                        acc.add(to_p(vv[t]), xr[t]);
+                        if (DV) dv_one(c + t, xr[t]);
                     }
                 }
                 return;
             }
+            if constexpr (CH == 2) {
+                const bool both = lim >= c + 2;
+                if (c < lx_end) {
+                    acc.add_two(to_p(vv[0]), xr[0], to_p(vv[1]), xr[1], both);
+                    if (DV) {
+                        if (both)
+                            dv_two(c, xr[0], xr[1]);
+                        else
+                            dv_one(c, xr[0]);
+                    }
+                    if (next_end == c + 1) {
+                        end_row(c + 1);
+                        if (c + 1 < lx_end) {
+                            acc.set(to_p(vv[1]), xr[1]);
+                            if (DV) dv_one(c + 1, xr[1]);
+                        }
+                    }
+                    if (next_end == c + 2) end_row(c + 2);
+                }
+            } else {
 #pragma unroll
-            for (int t = 0; t < CH; ++t) {
-                const int e = c + t;
-                if (e < lx_end) {
-                    end_rows(e);
-                    acc.add(to_p(vv[t]), xr[t]);
-                    if (DV) dv_step(t, e, xr);
+                for (int t = 0; t < CH; ++t) {
+                    if (c + t < lx_end) {
+                        acc.add(to_p(vv[t]), xr[t]);
+                        if (DV) dv_one(c + t, xr[t]);
+                        if (next_end == c + t + 1) end_row(c + t + 1);
+                    }
                 }
             }
+            __syncwarp();
         };
         if constexpr (STAGEP) {
-            // products of nonzero i (relative to the tile) at s_prod[i * VW]
+            // products of the tile's nonzero i at s_prod[i * VW]
             P* s_prod = reinterpret_cast<P*>(ws + prod_offset);
             {
                 int cidx[NJ];
 #pragma unroll
                 for (int j = 0; j < NJ; ++j) {
                     const int i = lane + 32 * j;
-                    cidx[j] = i < nz ? s_col[col_o + i] : 0;
+                    cidx[j] = i < nz ? col_t[x0 + i] : 0;
                 }
-                X xr[NJ][VW];
+                XRow<X, VW> xr[NJ];
 #pragma unroll
                 for (int j = 0; j < NJ; ++j)
-                    if (lane + 32 * j < nz) ld_vec<VW>(xm + (size_t)cidx[j] * d.ldx, xr[j]);
+                    if (lane + 32 * j < nz)
+                        xr[j].load(reinterpret_cast<const X*>(
+                            xl + (unsigned long long)(unsigned)cidx[j] * xstep));
 #pragma unroll
                 for (int j = 0; j < NJ; ++j) {
                     const int i = lane + 32 * j;
                     if (i < nz) {
-                        const P av = to_p(s_val[val_o + i]);
+                        const P av = to_p(val_t[x0 + i]);
 #pragma unroll
                         for (int v = 0; v < VW; ++v) s_prod[(size_t)i * VW + v] = av * (P)xr[j][v];
                     }
@@ -467,29 +832,44 @@ struct SpmmTile {
             }
             __syncwarp();
             for (int e = lx; e < lx_end; ++e) {
-                end_rows(e);
                 P pv[VW];
 #pragma unroll
-                for (int v = 0; v < VW; ++v) pv[v] = s_prod[(size_t)e * VW + v];
+                for (int v = 0; v < VW; ++v) pv[v] = s_prod[(size_t)(e - x0) * VW + v];
                 acc.add_p(pv);
+                if (next_end == e + 1) end_row(e + 1);
             }
         } else {
-            if (lx < lx_end) load_chunk(lx, xa, va);
-            for (int c = lx; c < lx_end; c += 2 * CH) {
-                if (c + CH < lx_end) load_chunk(c + CH, xb, vb);
+            // as many steps for every lane: the longest segment's
+            const int steps = __reduce_max_sync(0xFFFFFFFFu, (lx_end - lx + 2 * CH - 1) / (2 * CH));
+            int c = lx;
+            if (steps > 0) load_chunk(c, xa, va);
+            for (int i = 0; i < steps; ++i) {
+                load_chunk(c + CH, xb, vb);
                 consume(c, xa, va);
-                if (c + CH >= lx_end) break;
-                if (c + 2 * CH < lx_end) load_chunk(c + 2 * CH, xa, va);
+                load_chunk(c + 2 * CH, xa, va);
                 consume(c + CH, xb, vb);
+                c += 2 * CH;
             }
         }
-        while (ly < ly_end) {
-            emit(ly);
-            ++ly;
+
+        // ---- rows without nonzeros, G at a time
+        for (int r0 = 0; r0 < nr; r0 += 32) {
+            const int rl = r0 + lane;
+            const unsigned m =
+                __ballot_sync(0xFFFFFFFFu, rl < nr && rp_t[min(rl, nr - 1) + 1] == rp_t[min(rl, nr - 1)]);
+            if (m == 0u) continue;
+            for (int i = g; i < 32; i += G) {
+                if ((m >> i) & 1u) {
+                    double zero[VW];
+#pragma unroll
+                    for (int v = 0; v < VW; ++v) zero[v] = 0.0;
+                    finish_row(y0 + r0 + i, zero);
+                }
+            }
         }
 
         // ---- group segmented scan, per RHS column (stride LPG lanes)
-        int f = first_row >= 0;
+        int f = any_end;
         double sv[VW];
 #pragma unroll
         for (int v = 0; v < VW; ++v) sv[v] = acc.value(v);
@@ -515,34 +895,42 @@ struct SpmmTile {
         }
         const int rs = s_rp[rpo];
         const bool need_lb = nr > 0 && rs < x0;
-        const bool holds_first = first_row == 0 && need_lb;
+        const bool holds_first = had_open && first_row == 0 && need_lb;
+        AccRow<Acc, VW, P, X> first;
+        first.zero();
+        if (had_open) first.unstash(s_first, lane);
         double rv[VW];
 #pragma unroll
-        for (int v = 0; v < VW; ++v) rv[v] = ev[v] + first_val[v];
-        if (first_row >= 0 && !holds_first) {
-#pragma unroll
-            for (int v = 0; v < VW; ++v)
-                st_row(ym, (size_t)(y0 + first_row) * d.ldy + j0 + v, rv[v], alpha, beta);
-        }
+        for (int v = 0; v < VW; ++v) rv[v] = ev[v] + first.value(v);
+        if (had_open && !holds_first) finish_row(y0 + first_row, rv);
 
-        // ---- the tile's trailing partial (last group): published, and
-        // swapped with the next tile when the row began in this tile
+        // ---- the tile's trailing partial (last group).  Row y1 ends in tile
+        // lt_end: if it began in this tile and ends in the next, the two swap
+        // their partials; if it spans more tiles, the partial is published for
+        // the look-back of the tile it ends in.  The words that this launch
+        // uses are emptied in the other parity, for the next launch: which
+        // they are depends on the matrix and the tile size alone.
         const size_t par = (size_t)(epoch & 1u) * nslots;
-        if (g == G - 1) {
+        const size_t other = (size_t)((epoch + 1u) & 1u) * nslots;
+        if (g == G - 1 && y1 < nrow && lt + 1 < d.num_tiles) {
+            const bool began_here = rp_t[nr] >= x0 && rp_t[nr] < x1;
+            const int lt_end = (int)(((long long)rp_t[nr + 1] + y1) / ITEMS);
+            if (began_here && lt_end == lt + 1) {
+                const size_t w = (size_t)(u + 1) * K + j0;
 #pragma unroll
-            for (int v = 0; v < VW; ++v)
-                st_relaxed_u64(slots + par + (size_t)u * K + j0 + v, dbits(sv[v]));
-            if (y1 < d.nrow && lt + 1 < d.num_tiles) {
-                const int rs1 = s_rp[rpo + nr];
-                if (rs1 >= x0 && rs1 < x1) {
+                for (int v = 0; v < VW; ++v) {
+                    st_relaxed_u64(xch + other + w + v, kEmpty);
+                    const unsigned long long o = atomicExch(xch + par + w + v, dbits(sv[v]));
+                    if (o != kEmpty)
+                        st_row(y_row(y1), v,
+                               sv[v] + __longlong_as_double((long long)o), alpha, beta);
+                }
+            } else if (rp_t[nr] < x1) {  // (a row that starts at x1 has nothing here)
+                const size_t w = (size_t)u * K + j0;
 #pragma unroll
-                    for (int v = 0; v < VW; ++v) {
-                        const unsigned long long o =
-                            atomicExch(xch + par + (size_t)(u + 1) * K + j0 + v, dbits(sv[v]));
-                        if (o != kEmpty)
-                            st_row(ym, (size_t)y1 * d.ldy + j0 + v,
-                                   sv[v] + __longlong_as_double((long long)o), alpha, beta);
-                    }
+                for (int v = 0; v < VW; ++v) {
+                    st_relaxed_u64(slots + other + w + v, kEmpty);
+                    st_relaxed_u64(slots + par + w + v, dbits(sv[v]));
                 }
             }
         }
@@ -556,78 +944,32 @@ struct SpmmTile {
                         const unsigned long long o =
                             atomicExch(xch + par + (size_t)u * K + j0 + v, dbits(rv[v]));
                         if (o != kEmpty)
-                            st_row(ym, (size_t)y0 * d.ldy + j0 + v,
+                            st_row(y_row(y0), v,
                                    __longlong_as_double((long long)o) + rv[v], alpha, beta);
                     }
                 }
             } else {
-                // fixed-order look-back over the tiles back to the one that
-                // holds the row start.  Lane l serves column l % K; a step
-                // covers TPS * R tiles (tile offset l / K + TPS * r from
-                // `base`), all loaded before any is summed, so a row spanning
-                // hundreds of tiles takes few dependent round trips.  The
-                // summation order depends only on the tile and the row start.
-                constexpr int TPS = 32 / K > 0 ? 32 / K : 1;
-                constexpr int R = 8;
-                const bool lane_valid = lane < TPS * K;
-                double tot = 0.0;  // column (lane % K) of the sum
-                int base = lt - 1;
-                for (;;) {
-                    int tq[R];
-                    int first = INT_MAX;  // smallest offset of a tile starting at or before rs
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const int o = lane / K + TPS * r;
-                        tq[r] = base - o;
-                        if (lane_valid && (tq[r] < 0 || d.coords[tq[r]].x <= rs)) first = min(first, o);
-                    }
-                    first = __reduce_min_sync(0xFFFFFFFFu, first);
-                    unsigned long long bits[R];
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const int o = lane / K + TPS * r;
-                        bits[r] = 0ull;  // +0.0
-                        if (lane_valid && tq[r] >= 0 && o <= first)
-                            bits[r] = ld_relaxed_u64(slots + par + (size_t)(d.tile_begin + tq[r]) * K + (lane % K));
-                    }
-                    double c = 0.0;
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const int o = lane / K + TPS * r;
-                        if (lane_valid && tq[r] >= 0 && o <= first) {
-                            if (bits[r] == kEmpty) {
-                                const unsigned long long* p =
-                                    slots + par + (size_t)(d.tile_begin + tq[r]) * K + (lane % K);
-                                const unsigned long long t0 = global_timer_ns();
-                                while ((bits[r] = ld_relaxed_u64(p)) == kEmpty) {
-                                    __nanosleep(32);
-                                    if (*(volatile int*)&st->error != 0) break;
-                                    if (global_timer_ns() - t0 > kCarryWaitNs) {
-                                        atomicExch(&st->error, (int)MERBIT_ERR_TIMEOUT);
-                                        break;
-                                    }
-                                }
-                            }
-                            c += bits[r] == kEmpty ? 0.0 : __longlong_as_double((long long)bits[r]);
-                        }
-                    }
-                    // sum over the step's tiles, per column (lanes l, l+K, ...)
-#pragma unroll
-                    for (int o = K; o < 32; o <<= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-                    tot += c;
-                    if (first != INT_MAX) break;
-                    base -= TPS * R;
+                if (nlb == kSpmmLookBacks) {  // warp-uniform
+                    drain_spmm_look_backs<K, Y>(lbq, nlb, a, epoch, lane);
+                    nlb = 0;
                 }
-                double tv[VW];
-#pragma unroll
-                for (int v = 0; v < VW; ++v) tv[v] = __shfl_sync(0xFFFFFFFFu, tot, j0 + v);
                 if (holds_first) {
 #pragma unroll
                     for (int v = 0; v < VW; ++v)
-                        st_row(ym, (size_t)y0 * d.ldy + j0 + v, tv[v] + rv[v], alpha, beta);
+                        st_relaxed_u64(xch + par + (size_t)u * K + j0 + v, dbits(rv[v]));
                 }
+                if (lane == 0) {
+                    SpmmLookBack e;
+                    e.y = y_row(y0);
+                    e.head = u;
+                    // the row's first nonzero is item rs + y0 of the merge path
+                    e.first = d.tile_begin + (int)(((long long)rs + y0) / ITEMS);
+                    lbq[nlb] = e;
+                }
+                ++nlb;
             }
         }
+        __syncwarp();
     }
 };
 
@@ -644,13 +986,24 @@ struct SpmmStage {
 
 // ITEMS2 != 0: a batch whose matrices take tiles of either size; descriptor
 // field `ipt` holds the tile items of its matrix (0 or ITEMS: ITEMS).
+//
+// Resident CTAs of 4 warps per SM that the registers must allow: 5 (96
+// registers).  On Zipf-1M FP32 at k = 16 the forward ran 427, 351 and 373 us
+// at 4, 5 and 6, and without a bound (80 registers, spills) 367.  FP64 with the
+// fused dval, with two tile sizes or with 8 scalar gathers ahead would spill
+// at 5.
+template <int DT, int VW, int ITEMS2, bool DV>
+constexpr int kSpmmMinCtas = DT == MERBIT_F64 && (DV || ITEMS2 != 0 || VW == 1) ? 4 : 5;
+
 template <int DT, int K, int VW, int ITEMS, int ITEMS2, int WARPS, bool DV>
-__global__ void __launch_bounds__(WARPS * 32) spmm_kernel(const SpmmLaunch a) {
+__global__ void __launch_bounds__(WARPS * 32, kSpmmMinCtas<DT, VW, ITEMS2, DV>)
+    spmm_kernel(const SpmmLaunch a) {
     using St = SpmmStage<DT, K, VW, ITEMS, ITEMS2, DV>;
     using T = typename St::T1;
     using T2 = typename St::T2;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ unsigned s_epoch;
+    __shared__ SpmmLookBack s_lbq[WARPS][kSpmmLookBacks];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_epoch = *(volatile unsigned*)&a.state->epoch;
@@ -662,10 +1015,9 @@ __global__ void __launch_bounds__(WARPS * 32) spmm_kernel(const SpmmLaunch a) {
     }
     __syncthreads();
     const unsigned epoch = s_epoch;
-    reset_other_parity(a.slots, a.nslots, epoch);
-    reset_other_parity(a.xch, a.nslots, epoch);
     const int nw = (int)gridDim.x * WARPS;
     unsigned phase = 0;
+    int nlb = 0;  // queued look-backs of this warp
     int m = 0;  // matrix of the current tile (tiles are visited in increasing order)
     for (int u = (int)blockIdx.x * WARPS + warp; u < a.total_tiles; u += nw) {
         const SpmmDesc* dp;
@@ -687,11 +1039,19 @@ __global__ void __launch_bounds__(WARPS * 32) spmm_kernel(const SpmmLaunch a) {
         __syncwarp();
         if (ok) {
             if (second)
-                T2::process(a, d, u, lt, epoch, ws, lane);
+                T2::process(a, d, u, lt, epoch, ws, lane, s_lbq[warp], nlb);
             else
-                T::process(a, d, u, lt, epoch, ws, lane);
+                T::process(a, d, u, lt, epoch, ws, lane, s_lbq[warp], nlb);
+        } else {  // nothing published: leave no word of an earlier launch behind
+            const size_t other = (size_t)((epoch + 1u) & 1u) * a.nslots;
+            if (lane < K) {
+                st_relaxed_u64(a.slots + other + (size_t)u * K + lane, kEmpty);
+                if (u + 1 < a.total_tiles)
+                    st_relaxed_u64(a.xch + other + (size_t)(u + 1) * K + lane, kEmpty);
+            }
         }
     }
+    drain_spmm_look_backs<K, typename T::Y>(s_lbq[warp], nlb, a, epoch, lane);
     __syncthreads();
     if (threadIdx.x == 0) finish_launch(a.state, epoch);
 }

@@ -1,0 +1,112 @@
+"""The SpMM walk at the places where its branches change: rows that end at,
+just before and just after the ends of lane-group segments and tiles, runs of
+empty rows, rows over several tiles (look-backs, more of them per warp than its
+queue holds), vector and scalar stores of Y, and alpha / beta on all of them.
+
+Tolerances as for every SpMM test (component-wise against the
+extended-precision oracle): 1e-13 for f64, 1e-6 for f32 / bf16 values."""
+import numpy as np
+import pytest
+import torch
+
+import merbit_b200 as mb
+from merbit_b200 import synth
+from merbit_b200.autograd import SparseMatrix
+from oracle import oracle as O
+from tests.helpers import csr_from_lengths, stored_values, to_cuda
+
+TOL = {"f64": 1e-13, "f32": 1e-6, "bf16": 1e-6}
+# merge items of a lane group's segment and of a tile (vector width 4)
+SEG = {4: 15, 8: 31, 16: 63, 32: 127}
+TILE = {4: 480, 8: 496, 16: 504, 32: 508}
+
+
+def _lengths(k):
+    s, t = SEG[k], TILE[k]
+    rng = np.random.default_rng(k)
+    return np.concatenate([
+        np.arange(s - 3, s + 3).repeat(9),           # row ends drift over segment ends
+        [s - 1] * 40,                                # every segment one whole row
+        np.arange(t - 2, t + 3).repeat(3),           # ... and over tile ends
+        [t - 1] * 4, [0] * (2 * t + 1), [1] * (t + 5),
+        [0, 3 * t, 0, 0, 2 * t - 1, 2 * t, 1, 2 * t + 1, 0],   # rows over three tiles
+        rng.integers(0, 3, 3 * t), [2] * t, [5 * t + 7], [0] * 40,
+    ]).astype(np.int64)
+
+
+def _matrix(k, seed=0):
+    return csr_from_lengths(_lengths(k), ncol=4000, seed=seed)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["f64", "f32", "bf16"])
+@pytest.mark.parametrize("k", [4, 8, 16, 32])
+@pytest.mark.parametrize("alpha,beta,pad", [(1.0, 0.0, 0), (1.0, 0.0, 1), (-0.5, 2.0, 4)])
+def test_rows_at_segment_and_tile_ends(dtype, k, alpha, beta, pad):
+    A = _matrix(k)
+    xy = np.float64 if dtype == "f64" else np.float32
+    X = synth.uniform(5, A.ncol * k).reshape(A.ncol, k).astype(xy)
+    Y0 = synth.uniform(6, A.nrow * (k + pad)).reshape(A.nrow, k + pad).astype(xy)
+    if beta == 0.0:
+        Y0[:, :k] = np.nan  # never read
+    plan = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
+    xd = torch.from_numpy(X).cuda()
+    yo, ya = O.spmm(A.row_ptr, A.col, stored_values(A, dtype), X, k=k, alpha=alpha)
+    want = yo + (beta * Y0[:, :k].astype(np.float64) if beta else 0.0)
+    scale = ya + abs(beta) * (np.abs(Y0[:, :k]) if beta else 0.0)
+    bits = None
+    for _ in range(3):  # launches of either slot parity give the same bits
+        Yd = torch.from_numpy(Y0).cuda()
+        plan.spmm(xd, Yd[:, :k], alpha=alpha, beta=beta)
+        got = Yd.cpu().numpy()
+        assert (np.abs(got[:, :k] - want) <= TOL[dtype] * np.maximum(scale, 1e-300)).all()
+        assert np.array_equal(got[:, k:], Y0[:, k:])  # columns beyond k untouched
+        assert bits is None or np.array_equal(got, bits, equal_nan=True)
+        bits = got
+    plan.check()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("k", [1, 2, 4, 8, 16, 32])
+def test_fused_backward_at_segment_and_tile_ends(dtype, k):
+    """The same rows as the columns of A (rows of the transpose plan)."""
+    B = _matrix(max(k, 4), seed=1)
+    rows = np.repeat(np.arange(B.nrow), np.diff(B.row_ptr))
+    order = np.lexsort((rows, B.col))
+    rp = np.zeros(B.ncol + 1, np.int32)
+    np.cumsum(np.bincount(B.col, minlength=B.ncol), out=rp[1:])
+    A = synth.CSR(rp, rows[order].astype(np.int32), B.vals[order], B.nrow)  # A = B^T
+    xy = np.float64 if dtype == "f64" else np.float32
+    G = synth.uniform(7, A.nrow * k).reshape(A.nrow, k).astype(xy)
+    X = synth.uniform(8, A.ncol * k).reshape(A.ncol, k).astype(xy)
+    M = SparseMatrix(*to_cuda(A, dtype), ncol=A.ncol)
+    dX, dv = M.backward_fused(torch.from_numpy(G).cuda(), torch.from_numpy(X).cuda())
+    v = stored_values(A, dtype)
+    do = O.spmm_t(A.row_ptr, A.col, v, G, A.ncol)
+    da = O.spmm_t(A.row_ptr, A.col, np.abs(v), np.abs(G), A.ncol)
+    assert (np.abs(dX.cpu().numpy() - do) <= TOL[dtype] * np.maximum(da, 1e-300)).all()
+    ar = np.repeat(np.arange(A.nrow), np.diff(A.row_ptr))
+    g64, x64 = G.astype(np.longdouble)[ar], X.astype(np.longdouble)[A.col]
+    want, scale = (g64 * x64).sum(1), np.abs(g64 * x64).sum(1)
+    # at most 32 products and their sums, each within one unit of the partial sums
+    eps = np.finfo(xy).eps
+    assert (np.abs(dv.cpu().numpy() - want) <= (k + 1) * eps * np.maximum(scale, 1e-300)).all()
+
+
+@pytest.mark.gpu
+def test_more_look_backs_than_a_warp_queues():
+    """Rows of 700 nonzeros (three tiles of 256 items at k = 1): every warp
+    completes more split rows than its queue of 8 holds."""
+    nrow, length, ncol = 44_000, 700, 5_000
+    rng = np.random.default_rng(4)
+    rp = (np.arange(nrow + 1) * length).astype(np.int32)
+    col = rng.integers(0, ncol, nrow * length, dtype=np.int32)
+    vals = rng.standard_normal(nrow * length).astype(np.float32)
+    A = synth.CSR(rp, col, vals.astype(np.float64), ncol)
+    X = synth.uniform(9, ncol).reshape(ncol, 1).astype(np.float32)
+    plan = mb.Plan(*to_cuda(A, "f32"), ncol=ncol)
+    Y = plan.spmm(torch.from_numpy(X).cuda())
+    yo, ya = O.spmm(A.row_ptr, A.col, vals, X, k=1)
+    assert (np.abs(Y.cpu().numpy() - yo.reshape(-1, 1)) <= 1e-6 * ya.reshape(-1, 1)).all()
+    plan.check()
