@@ -43,6 +43,8 @@ using BatchSmem = WarpSmem<typename Prec<DT>::V, typename Prec<DT>::P, MAXIPT, 3
 // Tile source of a batch member: its descriptor, copied to the warp's
 // shared memory when the warp reaches the matrix.
 struct BatchSrc {
+    static constexpr int kWalkUnroll = 32;
+    static constexpr bool kDrainInWalk = true;
     const SpmmDesc* d;  // shared memory
     const SpmmLaunch& a;
     __device__ __forceinline__ int2 coord(int u) const { return d->coords[u]; }
@@ -53,7 +55,6 @@ struct BatchSrc {
     __device__ __forceinline__ int nrow() const { return d->nrow; }
     __device__ __forceinline__ int nnz() const { return d->nnz; }
     __device__ __forceinline__ int num_tiles() const { return d->num_tiles; }
-    __device__ __forceinline__ const int2* coords() const { return d->coords; }
     __device__ __forceinline__ unsigned long long* slots() const { return a.slots; }
     __device__ __forceinline__ unsigned long long* xch() const { return a.xch; }
     __device__ __forceinline__ int nslots() const { return a.nslots; }
@@ -65,6 +66,7 @@ struct BatchSrc {
 // it: y[r] = fma(beta, y[r], alpha * v).
 template <typename Y>
 struct BatchRowStore {
+    static constexpr int kAhead = 1;  // rows are stored one by one
     Y* y;
     double alpha, beta;
     __device__ __forceinline__ void operator()(int r, double v) {
@@ -77,42 +79,44 @@ struct BatchRowStore {
 template <int DT, bool CG, int IPT, int MAXIPT>
 using BT = WarpTile<DT, IPT, CG, BatchSmem<DT, MAXIPT>>;
 
-// Issues (ISSUE) or processes the tile of `ipt` items per lane: a kernel
-// with stages for MAXIPT takes ipt in {7, 11} (11), {7, 11, 15} (15) or
-// {15, 19, 23} (23); the tuner only assigns those.
-template <int DT, bool CG, int MAXIPT, bool ISSUE, int IPT, class... A>
-__device__ __forceinline__ void run_ipt(A&&... args) {
-    if constexpr (ISSUE)
-        BT<DT, CG, IPT, MAXIPT>::issue(args...);
-    else
-        BT<DT, CG, IPT, MAXIPT>::process(args...);
-}
-template <int DT, bool CG, int MAXIPT, bool ISSUE, class... A>
-__device__ __forceinline__ void dispatch_ipt(int ipt, A&&... args) {
+// Processes the tile of `ipt` items per lane: a kernel with stages for MAXIPT
+// takes ipt in {7, 11} (11), {7, 11, 15} (15) or {15, 19, 23} (23); the tuner
+// only assigns those.
+template <int DT, bool CG, int MAXIPT, class... A>
+__device__ __forceinline__ void process_ipt(int ipt, A&&... args) {
     if constexpr (MAXIPT == 11) {
         if (ipt == 7)
-            run_ipt<DT, CG, MAXIPT, ISSUE, 7>(args...);
+            BT<DT, CG, 7, MAXIPT>::process(args...);
         else
-            run_ipt<DT, CG, MAXIPT, ISSUE, 11>(args...);
+            BT<DT, CG, 11, MAXIPT>::process(args...);
     } else if constexpr (MAXIPT == 15) {
         if (ipt == 7)
-            run_ipt<DT, CG, MAXIPT, ISSUE, 7>(args...);
+            BT<DT, CG, 7, MAXIPT>::process(args...);
         else if (ipt == 11)
-            run_ipt<DT, CG, MAXIPT, ISSUE, 11>(args...);
+            BT<DT, CG, 11, MAXIPT>::process(args...);
         else
-            run_ipt<DT, CG, MAXIPT, ISSUE, 15>(args...);
+            BT<DT, CG, 15, MAXIPT>::process(args...);
     } else {
         if (ipt == 15)
-            run_ipt<DT, CG, MAXIPT, ISSUE, 15>(args...);
+            BT<DT, CG, 15, MAXIPT>::process(args...);
         else if (ipt == 19)
-            run_ipt<DT, CG, MAXIPT, ISSUE, 19>(args...);
+            BT<DT, CG, 19, MAXIPT>::process(args...);
         else
-            run_ipt<DT, CG, MAXIPT, ISSUE, 23>(args...);
+            BT<DT, CG, 23, MAXIPT>::process(args...);
     }
 }
 
+// Resident CTAs per SM: what the stages leave room for, at most 32 warps (64
+// registers).
+template <int DT, int WARPS, int MAXIPT>
+constexpr int kBatchWarpCtas = []() constexpr {
+    const int room = (int)(200 * 1024 / (BatchSmem<DT, MAXIPT>::bytes * WARPS));
+    return room < 1 ? 1 : room < 32 / WARPS ? room : 32 / WARPS;
+}();
+
 template <int DT, int WARPS, bool CG, int CV, int MAXIPT>
-__global__ void __launch_bounds__(WARPS * 32) batch_warp_kernel(const SpmmLaunch a) {
+__global__ void __launch_bounds__(WARPS * 32, kBatchWarpCtas<DT, WARPS, MAXIPT>)
+    batch_warp_kernel(const SpmmLaunch a) {
     using S = BatchSmem<DT, MAXIPT>;
     using Y = typename Prec<DT>::Y;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -144,16 +148,21 @@ __global__ void __launch_bounds__(WARPS * 32) batch_warp_kernel(const SpmmLaunch
     BatchRowStore<Y> out{nullptr, a.alpha, a.beta};
     const BatchSrc src{&s_desc[warp], a};
     int m = -1;  // matrix whose descriptor s_desc[warp] holds
-    for (int u = (int)blockIdx.x * WARPS + warp; u < a.total_tiles; u += nw) {
+    int2 next = make_int2(0, 0);  // the next tile's coordinates, once fetched
+    bool fetched = false;
+    for (int u = (int)blockIdx.x * WARPS + warp;; u += nw) {
+        const bool done = u >= a.total_tiles;
         int mm = m < 0 ? 0 : m;
-        while (mm + 1 < a.ndesc && a.descs[mm + 1].tile_begin <= u) ++mm;
-        if (mm != m) {  // warp-uniform
-            if (m >= 0) {
-                resolve_swap(pa, out);
-                resolve_swap(pb, out);
-                drain_look_backs(src, epoch, s_lbq[warp], nlb, lane, out);
-                nlb = 0;
-            }
+        if (!done)
+            while (mm + 1 < a.ndesc && a.descs[mm + 1].tile_begin <= u) ++mm;
+        if (m >= 0 && (done || mm != m)) {  // warp-uniform
+            resolve_swap(pa, out);
+            resolve_swap(pb, out);
+            drain_look_backs(src, epoch, s_lbq[warp], nlb, lane, out);
+            nlb = 0;
+        }
+        if (done) break;
+        if (mm != m) {
             __syncwarp();
             constexpr int kWords = (int)(sizeof(SpmmDesc) / 4);
             static_assert(sizeof(SpmmDesc) % 4 == 0 && kWords <= 32, "descriptor copy");
@@ -166,18 +175,17 @@ __global__ void __launch_bounds__(WARPS * 32) batch_warp_kernel(const SpmmLaunch
         }
         const int lt = u - s_desc[warp].tile_begin;
         const int ipt = s_desc[warp].ipt;  // warp-uniform
-        dispatch_ipt<DT, CG, MAXIPT, true>(ipt, src, lt, ws, bar, lane);
+        if (!fetched) next = fetch_coords(src, lt, lane);
+        const TileCoords at = spread_coords(next);
+        BT<DT, CG, MAXIPT, MAXIPT>::issue(src, at, ws, bar, lane);  // the same for every ipt
+        fetched = lt + nw < s_desc[warp].num_tiles;
+        if (fetched) next = fetch_coords(src, lt + nw, lane);
         const bool ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(bar, phase, a.state));
         phase ^= 1u;
         __syncwarp();
         if (ok)
-            dispatch_ipt<DT, CG, MAXIPT, false>(ipt, src, lt, epoch, ws, lane, pa, pb, out,
-                                                s_lbq[warp], nlb);
-    }
-    if (m >= 0) {
-        resolve_swap(pa, out);
-        resolve_swap(pb, out);
-        drain_look_backs(src, epoch, s_lbq[warp], nlb, lane, out);
+            process_ipt<DT, CG, MAXIPT>(ipt, src, lt, at, epoch, ws, lane, pa, pb, out, s_lbq[warp],
+                                        nlb);
     }
     __syncthreads();
     if (threadIdx.x == 0) finish_launch(a.state, epoch);

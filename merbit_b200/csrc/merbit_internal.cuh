@@ -187,6 +187,39 @@ __device__ __forceinline__ double read_carry(const unsigned long long* slots, in
     }
 }
 
+// Loads the carries p[0], p[stride], ... (those at offsets below `left`; +0.0
+// for the others), all in flight together, waiting (bounded) until each is
+// published.
+template <int N>
+__device__ __forceinline__ void load_carries(unsigned long long (&b)[N],
+                                             const unsigned long long* p, int stride, int left,
+                                             LaunchState* st) {
+    bool missing = false;
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        b[r] = r * stride < left ? ld_relaxed_u64(p + r * stride) : 0ull;
+        missing = missing || b[r] == kEmpty;
+    }
+    if (!missing) return;
+    const unsigned long long t0 = global_timer_ns();
+    for (;;) {
+        __nanosleep(32);
+        missing = false;
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            if (b[r] == kEmpty) b[r] = ld_relaxed_u64(p + r * stride);
+            missing = missing || b[r] == kEmpty;
+        }
+        if (!missing) return;
+        const bool late = global_timer_ns() - t0 > kCarryWaitNs;
+        if (late) atomicExch(&st->error, (int)MERBIT_ERR_TIMEOUT);
+        if (late || *(volatile int*)&st->error != 0) break;
+    }
+#pragma unroll
+    for (int r = 0; r < N; ++r)
+        if (b[r] == kEmpty) b[r] = 0ull;
+}
+
 // Grid-strided refill of the other parity's slots.
 __device__ __forceinline__ void reset_other_parity(unsigned long long* slots, int nslots,
                                                    unsigned epoch) {
@@ -196,32 +229,33 @@ __device__ __forceinline__ void reset_other_parity(unsigned long long* slots, in
         o[i] = kEmpty;
 }
 
-// Decoupled look-back by one warp: the sum of the carries of tiles u-1,
-// u-2, ... down to the tile that contains nonzero index rs (the start of
-// the row that tile u completes first), in a fixed order -- 32 tiles per
-// step, butterfly reduction -- so the result does not depend on timing.
-// Tile t's carry is in slot slot_base + t (a batch places each matrix's
-// tiles at its own offset of one slot array).
-__device__ __forceinline__ double look_back(const int2* coords, const unsigned long long* slots,
-                                            int nslots, unsigned epoch, LaunchState* st, int u,
-                                            int rs, int lane, int slot_base = 0) {
-    double total = 0.0;
-    int base = u - 1;
-    for (;;) {
-        const int tq = base - lane;
-        const bool valid = tq >= 0;
-        const int cx = valid ? coords[tq].x : 0;
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, !valid || cx <= rs);
-        const int last = m ? __ffs(m) - 1 : 31;
-        double c = 0.0;
-        if (valid && lane <= last) c = read_carry(slots, nslots, epoch, slot_base + tq, st);
+// Decoupled look-back by one warp: the sum of the carries of tiles
+// [first, u), where `first` is the tile in which the row that tile u completes
+// first begins: its first nonzero rs is item rs + row of the merge path, so
+// first = (rs + row) / tile items, and no tile has to be read to find the one
+// before it.  Lane l takes tiles first + l, + 32, ...; kLookBackAhead of its
+// carries are loaded before the first is summed (a row of 200,000 nonzeros
+// spans 400 tiles: 4 round trips instead of 13), then a butterfly: the order
+// depends only on the tiles, not on timing.  Tile t's carry is in slot
+// slot_base + t (a batch places each matrix's tiles at its own offset of one
+// slot array).
+constexpr int kLookBackAhead = 4;
+
+__device__ __forceinline__ double look_back(const unsigned long long* slots, int nslots,
+                                            unsigned epoch, LaunchState* st, int first, int u,
+                                            int lane, int slot_base) {
+    const unsigned long long* p = slots + (size_t)(epoch & 1u) * nslots + slot_base;
+    double sum = 0.0;
+    for (int t = first + lane; t < u; t += 32 * kLookBackAhead) {
+        unsigned long long b[kLookBackAhead];
+        load_carries<kLookBackAhead>(b, p + t, 32, u - t, st);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-        total += c;
-        if (m) break;
-        base -= 32;
+        for (int r = 0; r < kLookBackAhead; ++r) sum += __longlong_as_double((long long)b[r]);
     }
-    return total;
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    return sum;
 }
 
 // ---------------------------------------------------------------------------
@@ -463,6 +497,8 @@ int spmv_launch(int dtype, int cfg, bool vec, const SpmvLaunch& a, cudaStream_t 
 // as stored to the thread's running residual.
 template <typename Y, bool RES>
 struct RowStore {
+    // rows per lane whose operands are loaded before the first is stored
+    static constexpr int kAhead = 4;
     Y* y;
     const Y* z;
     const Y* xres;
@@ -482,6 +518,25 @@ struct RowStore {
         const Y yo = (Y)o;
         y[r] = yo;
         if (RES) res += fabs((double)yo - (double)xres[r]);
+    }
+    // the same for N rows (r < 0: none): all loads before the first store
+    template <int N>
+    __device__ __forceinline__ void rows(const int (&r)[N], const double (&v)[N]) {
+        Y zr[N], xr[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            zr[i] = beta != 0.0 && r[i] >= 0 ? z[r[i]] : (Y)0;
+            xr[i] = RES && r[i] >= 0 ? xres[r[i]] : (Y)0;
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if (r[i] < 0) continue;
+            double o = __dmul_rn(alpha, v[i]);
+            if (beta != 0.0) o = __fma_rn(beta, (double)zr[i], o);
+            const Y yo = (Y)o;
+            y[r[i]] = yo;
+            if (RES) res += fabs((double)yo - (double)xr[i]);
+        }
     }
 };
 

@@ -412,26 +412,9 @@ __device__ __forceinline__ void spmm_look_back(const SpmmLookBack& e, unsigned l
     double sum = 0.0;
     for (int t = e.first + lane / K; t < e.head; t += TPS * R) {
         unsigned long long bits[R];
+        load_carries<R>(bits, slots + (size_t)t * K + j, TPS * K, (e.head - t) * K, st);
 #pragma unroll
-        for (int r = 0; r < R; ++r)
-            bits[r] = t + r * TPS < e.head ? ld_relaxed_u64(slots + (size_t)(t + r * TPS) * K + j) : 0ull;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            if (bits[r] == kEmpty) {  // not published yet: wait (bounded)
-                const unsigned long long* p = slots + (size_t)(t + r * TPS) * K + j;
-                const unsigned long long t0 = global_timer_ns();
-                while ((bits[r] = ld_relaxed_u64(p)) == kEmpty) {
-                    __nanosleep(32);
-                    if (*(volatile int*)&st->error != 0) break;
-                    if (global_timer_ns() - t0 > kCarryWaitNs) {
-                        atomicExch(&st->error, (int)MERBIT_ERR_TIMEOUT);
-                        break;
-                    }
-                }
-                if (bits[r] == kEmpty) bits[r] = 0ull;
-            }
-            sum += __longlong_as_double((long long)bits[r]);
-        }
+        for (int r = 0; r < R; ++r) sum += __longlong_as_double((long long)bits[r]);
     }
     __syncwarp();
 #pragma unroll
@@ -914,7 +897,7 @@ struct SpmmTile {
         const size_t other = (size_t)((epoch + 1u) & 1u) * nslots;
         if (g == G - 1 && y1 < nrow && lt + 1 < d.num_tiles) {
             const bool began_here = rp_t[nr] >= x0 && rp_t[nr] < x1;
-            const int lt_end = (int)(((long long)rp_t[nr + 1] + y1) / ITEMS);
+            const int lt_end = (int)((unsigned)(rp_t[nr + 1] + y1) / (unsigned)ITEMS);
             if (began_here && lt_end == lt + 1) {
                 const size_t w = (size_t)(u + 1) * K + j0;
 #pragma unroll
@@ -963,7 +946,7 @@ struct SpmmTile {
                     e.y = y_row(y0);
                     e.head = u;
                     // the row's first nonzero is item rs + y0 of the merge path
-                    e.first = d.tile_begin + (int)(((long long)rs + y0) / ITEMS);
+                    e.first = d.tile_begin + (int)((unsigned)(rs + y0) / (unsigned)ITEMS);
                     lbq[nlb] = e;
                 }
                 ++nlb;

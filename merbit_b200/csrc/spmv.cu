@@ -228,7 +228,8 @@ __global__ void __launch_bounds__(BLOCK) spmv_tile_kernel(const SpmvLaunch a) {
     // timing.
     const bool need_lb = nr > 0 && s_rp[0] < x0;
     if (need_lb && warp == 0) {
-        const double total = look_back(a.coords, a.slots, a.nslots, epoch, a.state, t, s_rp[0], lane);
+        const int first = (int)((unsigned)(s_rp[0] + y0) / (unsigned)D);
+        const double total = look_back(a.slots, a.nslots, epoch, a.state, first, t, lane, 0);
         if (lane == 0) s_carry = total;
     }
     __syncthreads();

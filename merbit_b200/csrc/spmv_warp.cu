@@ -5,12 +5,11 @@
 //
 //   1. lane 0 issues bulk async copies (cp.async.bulk through the TMA
 //      engine, L2 evict-first) of the tile's row_ptr window (none for a
-//      tile inside one row), col_idx slice and vals slice into one of the
-//      warp's STAGES shared-memory stages,
-//      completing on that stage's mbarrier.  Ranges are rounded out to 16
-//      bytes (only the last few elements of an array, which rounding would
-//      overrun, are fetched with plain loads).  With STAGES = 2 the next
-//      tile's copies are issued before the current tile is processed;
+//      tile inside one row), col_idx slice and vals slice into the warp's
+//      shared-memory stage, completing on its mbarrier.  Ranges are rounded
+//      out to 16 bytes (only the last few elements of an array, which rounding
+//      would overrun, are fetched with plain loads).  The coordinates of the
+//      next tile are loaded while the current one is processed;
 //   2. lanes gather x[col] for up to IPT nonzeros each (all loads in flight
 //      together) and overwrite the staged values with the products;
 //   3. each lane finds its segment start by merge search in shared memory
@@ -49,6 +48,8 @@ namespace merbit {
 // The tile source of a single-matrix launch: everything comes from the
 // kernel parameter block, and local tile u is slot u.
 struct SpmvSrc {
+    static constexpr int kWalkUnroll = 4;
+    static constexpr bool kDrainInWalk = false;
     const SpmvLaunch& a;
     __device__ __forceinline__ int2 coord(int u) const { return a.coords[u]; }
     __device__ __forceinline__ const int32_t* row_ptr() const { return a.row_ptr; }
@@ -58,7 +59,6 @@ struct SpmvSrc {
     __device__ __forceinline__ int nrow() const { return a.nrow; }
     __device__ __forceinline__ int nnz() const { return a.nnz; }
     __device__ __forceinline__ int num_tiles() const { return a.num_tiles; }
-    __device__ __forceinline__ const int2* coords() const { return a.coords; }
     __device__ __forceinline__ unsigned long long* slots() const { return a.slots; }
     __device__ __forceinline__ unsigned long long* xch() const { return a.xch; }
     __device__ __forceinline__ int nslots() const { return a.nslots; }
@@ -74,8 +74,17 @@ template <int DT, int IPT, bool FULL>
 using SpmvWarpSmem = WarpSmem<typename Prec<DT>::V, typename Prec<DT>::P, IPT,
                               FULL ? 32 * IPT + 16 : warp_rp_cap(IPT)>;
 
-template <int DT, int WARPS, int IPT, int STAGES, bool RES, bool CG, int CV, bool FULL>
-__global__ void __launch_bounds__(WARPS * 32) spmv_warp_kernel(const SpmvLaunch a) {
+// Resident CTAs per SM: what the stages leave room for, at most 32 warps (64
+// registers).
+template <int DT, int WARPS, int IPT, bool FULL>
+constexpr int kSpmvWarpCtas = []() constexpr {
+    const int room = (int)(200 * 1024 / (SpmvWarpSmem<DT, IPT, FULL>::bytes * WARPS));
+    return room < 1 ? 1 : room < 32 / WARPS ? room : 32 / WARPS;
+}();
+
+template <int DT, int WARPS, int IPT, bool RES, bool CG, int CV, bool FULL>
+__global__ void __launch_bounds__(WARPS * 32, kSpmvWarpCtas<DT, WARPS, IPT, FULL>)
+    spmv_warp_kernel(const SpmvLaunch a) {
     using T = WarpTile<DT, IPT, CG, SpmvWarpSmem<DT, IPT, FULL>>;
     using S = typename T::S;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -84,13 +93,10 @@ __global__ void __launch_bounds__(WARPS * 32) spmv_warp_kernel(const SpmvLaunch 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_epoch = *(volatile unsigned*)&a.state->epoch;
-    // stage k of this warp: wbase + k * S::bytes, its barrier at bar_offset;
-    // bit k of `phases` is the parity stage k waits for next
-    unsigned char* wbase = smem + (size_t)warp * STAGES * S::bytes;
+    unsigned char* ws = smem + (size_t)warp * S::bytes;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(ws + S::bar_offset);
     if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < STAGES; ++k)
-            mbar_init(reinterpret_cast<uint64_t*>(wbase + k * S::bytes + S::bar_offset), 1);
+        mbar_init(bar, 1);
         fence_mbar_init();
     }
     __syncthreads();
@@ -98,7 +104,7 @@ __global__ void __launch_bounds__(WARPS * 32) spmv_warp_kernel(const SpmvLaunch 
     reset_other_parity(a.slots, a.nslots, epoch);
     reset_other_parity(a.xch, a.nslots, epoch);
     const int nw = (int)gridDim.x * WARPS;
-    unsigned phases = 0u;
+    unsigned phase = 0u;
     RowStore<typename T::Y, RES> out(a);
     int nlb = 0;  // queued look-backs of this warp
     PendingSwap pa, pb;
@@ -109,27 +115,28 @@ __global__ void __launch_bounds__(WARPS * 32) spmv_warp_kernel(const SpmvLaunch 
     pb.carry = 0;
     const SpmvSrc src{a};
     int u = (int)blockIdx.x * WARPS + warp;
-    if (u < a.num_tiles)
-        T::issue(src, u, wbase, reinterpret_cast<uint64_t*>(wbase + S::bar_offset), lane);
-    int k = 0;
-    for (; u < a.num_tiles; u += nw) {
+    TileCoords at = {};
+    if (u < a.num_tiles) {
+        at = spread_coords(fetch_coords(src, u, lane));
+        T::issue(src, at, ws, bar, lane);
+    }
+    while (u < a.num_tiles) {
         const int un = u + nw;
-        unsigned char* cur = wbase + (size_t)k * S::bytes;
-        uint64_t* cbar = reinterpret_cast<uint64_t*>(cur + S::bar_offset);
-        if (STAGES == 2 && un < a.num_tiles) {
-            unsigned char* nxt = wbase + (size_t)(k ^ 1) * S::bytes;
-            T::issue(src, un, nxt, reinterpret_cast<uint64_t*>(nxt + S::bar_offset), lane);
-        }
-        const bool ok =
-            __all_sync(0xFFFFFFFFu, mbar_wait_bounded(cbar, (phases >> k) & 1u, a.state));
-        phases ^= 1u << k;
+        int2 next = make_int2(0, 0);
+        if (un < a.num_tiles) next = fetch_coords(src, un, lane);
+        const bool ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(bar, phase, a.state));
+        phase ^= 1u;
         __syncwarp();
-        if (ok) T::process(src, u, epoch, cur, lane, pa, pb, out, s_lbq[warp], nlb);
-        if (STAGES == 1) {
-            if (un < a.num_tiles) T::issue(src, un, cur, cbar, lane);
-        } else {
-            k ^= 1;
+        if (ok) T::process(src, u, at, epoch, ws, lane, pa, pb, out, s_lbq[warp], nlb);
+        if (nlb == kLookBackQueue) {  // warp-uniform
+            drain_look_backs(src, epoch, s_lbq[warp], nlb, lane, out);
+            nlb = 0;
         }
+        if (un < a.num_tiles) {
+            at = spread_coords(next);
+            T::issue(src, at, ws, bar, lane);
+        }
+        u = un;
     }
     resolve_swap(pa, out);
     resolve_swap(pb, out);
@@ -196,19 +203,19 @@ int launch_coop(K kern, int warps, size_t smem, int carveout, int* grid_cap, con
     return e == cudaSuccess ? (int)MERBIT_OK : cuda_fail(e, name);
 }
 
-template <int DT, int WARPS, int IPT, int STAGES, bool RES, bool CG, int CV, bool FULL>
+template <int DT, int WARPS, int IPT, bool RES, bool CG, int CV, bool FULL>
 int launch_warp_k(const SpmvLaunch& a, cudaStream_t s) {
     using S = SpmvWarpSmem<DT, IPT, FULL>;
     static int grid_cap[64] = {};
     if (RES && !a.partials) return fail(MERBIT_ERR_INVALID, "spmv_warp: residual without partials");
-    return launch_coop(spmv_warp_kernel<DT, WARPS, IPT, STAGES, RES, CG, CV, FULL>, WARPS,
-                       S::bytes * WARPS * STAGES, CV, grid_cap, a, s, "spmv_warp_kernel");
+    return launch_coop(spmv_warp_kernel<DT, WARPS, IPT, RES, CG, CV, FULL>, WARPS,
+                       S::bytes * WARPS, CV, grid_cap, a, s, "spmv_warp_kernel");
 }
 
-template <int DT, int WARPS, int IPT, int STAGES, bool CG, int CV, bool FULL = false>
+template <int DT, int WARPS, int IPT, bool CG, int CV, bool FULL = false>
 int launch_warp(const SpmvLaunch& a, cudaStream_t s) {
-    return a.residual ? launch_warp_k<DT, WARPS, IPT, STAGES, true, CG, CV, FULL>(a, s)
-                      : launch_warp_k<DT, WARPS, IPT, STAGES, false, CG, CV, FULL>(a, s);
+    return a.residual ? launch_warp_k<DT, WARPS, IPT, true, CG, CV, FULL>(a, s)
+                      : launch_warp_k<DT, WARPS, IPT, false, CG, CV, FULL>(a, s);
 }
 
 // The (warps, items per thread, gather hint, carveout) combinations of the
@@ -219,10 +226,10 @@ int launch_warp_dt(const SpmvConfig& c, const SpmvLaunch& a, cudaStream_t s) {
     if (c.stages != 1) return fail(MERBIT_ERR_INVALID, "spmv_warp: no such configuration");
 #define MERBIT_WARP_CASE(W, I, G, C)                                                   \
     if (warps == W && ipt == I && c.cg == G && c.carveout == C && !c.stg)              \
-        return launch_warp<DT, W, I, 1, G, C>(a, s);
+        return launch_warp<DT, W, I, G, C>(a, s);
 #define MERBIT_WARP_FULL_CASE(W, I, G, C)                                              \
     if (warps == W && ipt == I && c.cg == G && c.carveout == C && c.stg)               \
-        return launch_warp<DT, W, I, 1, G, C, true>(a, s);
+        return launch_warp<DT, W, I, G, C, true>(a, s);
     MERBIT_WARP_CASE(8, 15, 1, kCarveoutL1)
     MERBIT_WARP_CASE(4, 15, 1, kCarveoutL1)
     MERBIT_WARP_CASE(8, 11, 1, kCarveoutL1)

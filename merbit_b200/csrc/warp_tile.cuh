@@ -9,6 +9,13 @@
 //   row_ptr(), col(), vals(), x(), nrow(), nnz(), num_tiles()
 //   slots(), xch(), nslots(), state()   the launch's slot arrays and state
 //   slot_base()     slot index of local tile 0
+//   kWalkUnroll     steps of the walk per loop iteration
+//   kDrainInWalk    whether process() empties a full look-back queue itself (else
+//                   the kernel does, between tiles)
+// The last two only place code.  Measured (us): a single matrix with 4 steps
+// per iteration and the queue emptied between tiles, Zipf-1.1M BF16 118
+// against 126 with both as in the batch; the batch, 64 R-MAT matrices FP32, with
+// the walk unrolled and the queue emptied inside, 488 against 500.
 // so that one tile walk serves a single matrix and the matrices of a batch.
 #pragma once
 
@@ -30,12 +37,17 @@ constexpr int kWarpBlockSum = std::is_same<Acc, AccTwoSum>::value ? 4 : 1;
 // One stage of a warp: row_ptr window (RP entries; warp_rp_cap(IPT) by
 // default -- the plan only runs such a configuration when no tile ends more
 // rows than fit), col slice and value slice (W + rounding), one mbarrier.
-// Completed rows are staged for the coalesced write in whichever slice is
-// dead after the products are formed: the col slice when products
-// overwrite the values, the value slice when they overwrite the columns
-// (bf16); rows beyond OUTCAP go straight to y.  W is the largest tile the
-// stage holds (a batch sizes one stage for the largest items per lane of
-// its matrices).
+// Completed rows are staged for the coalesced write: the first OUTCAP in the
+// slice that is dead after the products are formed (the col slice when
+// products overwrite the values, the value slice when they overwrite the
+// columns: bf16), the others behind the products.  A tile of nr row ends has
+// nr places fewer for products, so with products in the value slice all its
+// rows fit; with bf16 the rows beyond both go straight to y.  (With one slice
+// only, tiles of empty and one-entry rows wrote most of their rows from inside
+// the walk, one dependent load of z and x after another: PageRank on a
+// 400,000-node R-MAT graph took 74 us a step.)  W is the largest tile the stage
+// holds (a batch sizes one stage for the largest items per lane of its
+// matrices).
 template <typename V, typename P, int IPT, int RP = warp_rp_cap(IPT)>
 struct WarpSmem {
     static constexpr int W = 32 * IPT;
@@ -45,8 +57,9 @@ struct WarpSmem {
     static constexpr size_t val_bytes = align16((size_t)CAP * sizeof(V));
     static constexpr bool prod_in_val = sizeof(P) == sizeof(V);
     static constexpr size_t out_offset = prod_in_val ? rp_bytes : rp_bytes + col_bytes;
-    static constexpr int OUTCAP_ = (int)((prod_in_val ? col_bytes : val_bytes) / 8);
-    static constexpr int OUTCAP = OUTCAP_ < 256 ? OUTCAP_ : 256;
+    static constexpr int OUTCAP = (int)((prod_in_val ? col_bytes : val_bytes) / 8);
+    // bytes of the slice that holds the products
+    static constexpr size_t prod_bytes = prod_in_val ? val_bytes : col_bytes;
     static constexpr size_t bar_offset = rp_bytes + col_bytes + val_bytes;
     static constexpr size_t bytes = bar_offset + 16;
 };
@@ -111,9 +124,11 @@ __device__ __forceinline__ void resolve_swap(PendingSwap& p, RS& out) {
 // on other warps at about the same time.  Its look-back is queued and taken
 // later (when the queue is full, else after the warp's last tile), so the
 // warp does not wait for those tiles while it still has tiles to process.
+// A tile queues at most one.
 struct LookBack {
     double head;  // the completing tile's part of the row
-    int row, u, rs;
+    int row, u;
+    int first;    // the tile in which the row begins
 };
 constexpr int kLookBackQueue = 8;
 
@@ -122,8 +137,8 @@ __device__ __forceinline__ void drain_look_backs(const Src& src, unsigned epoch,
                                                  const LookBack* q, int n, int lane, RS& out) {
     for (int i = 0; i < n; ++i) {
         const LookBack e = q[i];
-        const double total = look_back(src.coords(), src.slots(), src.nslots(), epoch, src.state(),
-                                       e.u, e.rs, lane, src.slot_base());
+        const double total = look_back(src.slots(), src.nslots(), epoch, src.state(), e.first, e.u,
+                                       lane, src.slot_base());
         if (lane == 0) out(e.row, total + e.head);
     }
     __syncwarp();
@@ -135,6 +150,26 @@ __device__ __forceinline__ void drain_look_backs(const Src& src, unsigned epoch,
 template <bool CG, typename T>
 __device__ __forceinline__ T gather_x(const T* p) {
     return CG ? __ldcg(p) : __ldg(p);
+}
+
+// Merge-path coordinates a tile needs: where it starts and ends, and where the
+// tile before it starts.  A warp loads those of its next tile (one per lane 0
+// to 2) before it processes the current one, so that their latency does not
+// come before the next tile's copies, and broadcasts them when it gets there.
+struct TileCoords {
+    int2 c0, c1;
+    int prev_x;
+};
+template <class Src>
+__device__ __forceinline__ int2 fetch_coords(const Src& src, int u, int lane) {
+    return lane < 3 ? src.coord(max(u - 1 + lane, 0)) : make_int2(0, 0);
+}
+__device__ __forceinline__ TileCoords spread_coords(int2 c) {
+    TileCoords t;
+    t.prev_x = __shfl_sync(0xFFFFFFFFu, c.x, 0);
+    t.c0 = make_int2(__shfl_sync(0xFFFFFFFFu, c.x, 1), __shfl_sync(0xFFFFFFFFu, c.y, 1));
+    t.c1 = make_int2(__shfl_sync(0xFFFFFFFFu, c.x, 2), __shfl_sync(0xFFFFFFFFu, c.y, 2));
+    return t;
 }
 
 // One warp tile of IPT items per lane.  Src is where the tile's matrix comes
@@ -158,13 +193,12 @@ struct WarpTile {
     // enter in blocks of this many, fused in f32 (1: one TwoSum each)
     static constexpr int kBlockSum = kWarpBlockSum<Acc>;
 
-    // Issues the copies of tile u into stage `ws`; lane 0 arms the barrier
-    // with the byte count before any copy is issued.
+    // Issues the copies of the tile at `at` into stage `ws`; lane 0 arms the
+    // barrier with the byte count before any copy is issued.
     template <class Src>
-    static __device__ __forceinline__ void issue(const Src& src, int u, unsigned char* ws,
-                                                 uint64_t* bar, int lane) {
-        const int2 c0 = src.coord(u);
-        const int2 c1 = src.coord(u + 1);
+    static __device__ __forceinline__ void issue(const Src& src, const TileCoords& at,
+                                                 unsigned char* ws, uint64_t* bar, int lane) {
+        const int2 c0 = at.c0, c1 = at.c1;
         int* s_rp = reinterpret_cast<int*>(ws);
         int* s_col = reinterpret_cast<int*>(ws + S::rp_bytes);
         V* s_val = reinterpret_cast<V*>(ws + S::rp_bytes + S::col_bytes);
@@ -192,19 +226,16 @@ struct WarpTile {
 
     // Processes tile u from stage `ws` (its copies complete).
     template <class Src, class RS>
-    static __device__ __forceinline__ void process(const Src& src, int u, unsigned epoch,
-                                                   unsigned char* ws, int lane,
+    static __device__ __forceinline__ void process(const Src& src, int u, const TileCoords& at,
+                                                   unsigned epoch, unsigned char* ws, int lane,
                                                    PendingSwap& pa, PendingSwap& pb, RS& out,
                                                    LookBack* lbq, int& nlb) {
         const int* s_rp = reinterpret_cast<const int*>(ws);
         const int* s_col = reinterpret_cast<const int*>(ws + S::rp_bytes);
         const V* s_val = reinterpret_cast<const V*>(ws + S::rp_bytes + S::col_bytes);
-        double* s_out = reinterpret_cast<double*>(ws + S::out_offset);
 
-        const int2 c0 = src.coord(u);
-        const int2 c1 = src.coord(u + 1);
-        const int prev_x = u > 0 ? src.coord(u - 1).x : 0;
-        const int x0 = c0.x, y0 = c0.y, x1 = c1.x, y1 = c1.y;
+        const int prev_x = at.prev_x;
+        const int x0 = at.c0.x, y0 = at.c0.y, x1 = at.c1.x, y1 = at.c1.y;
         const int nz = x1 - x0, nr = y1 - y0, L = nz + nr;
         const int rp_base = y0 & ~3, col_base = x0 & ~3, val_base = x0 & ~(GV - 1);
 
@@ -299,6 +330,19 @@ struct WarpTile {
         }
         __syncwarp();
 
+        // ---- where completed rows wait: row r at place(r), r < out_cap (the
+        // first slice alone when a row's store loads nothing, RS::kAhead = 1:
+        // rows beyond it may as well go straight to y, in fewer instructions)
+        double* s_out = reinterpret_cast<double*>(ws + S::out_offset);
+        constexpr bool kStageAll = RS::kAhead > 1;
+        const int used = ((x0 - pbase + nz) * (int)sizeof(P) + 7) & ~7;  // products
+        double* s_more = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(s_prod) + used) -
+                         kOutCap;
+        const int out_cap = !kStageAll        ? kOutCap
+                            : S::prod_in_val ? INT_MAX
+                                             : kOutCap + ((int)S::prod_bytes - used) / 8;
+        auto place = [&](int r) { return (!kStageAll || r < kOutCap ? s_out : s_more) + r; };
+
         // ---- this lane's segment: merge search in the staged row_ptr window
         const int rpo = y0 - rp_base;
         const int pofs = x0 - pbase;
@@ -323,7 +367,7 @@ struct WarpTile {
         int first_row = -1;
         double first_val = 0.0;
         int next_end = ly < nr ? s_rp[rpo + ly + 1] - x0 : INT_MAX;
-#pragma unroll
+#pragma unroll Src::kWalkUnroll
         for (int i = 0; i < IPT; ++i) {
             const bool valid = dl + i < L;
             const bool is_end = valid && lx >= next_end;
@@ -334,8 +378,8 @@ struct WarpTile {
                 if (first_row < 0) {
                     first_row = ly;
                     first_val = v;
-                } else if (ly < kOutCap) {
-                    s_out[ly] = v;
+                } else if (ly < out_cap) {
+                    *place(ly) = v;
                 } else {
                     out(y0 + ly, v);
                 }
@@ -374,8 +418,8 @@ struct WarpTile {
         const double rv = ev + first_val;   // this lane's first completed row
         const bool holds_first = first_row == 0 && need_lb;
         if (first_row >= 0 && !holds_first) {
-            if (first_row < kOutCap)
-                s_out[first_row] = rv;
+            if (first_row < out_cap)
+                *place(first_row) = rv;
             else
                 out(y0 + first_row, rv);
         }
@@ -400,9 +444,25 @@ struct WarpTile {
 
         // ---- coalesced write of the staged rows (row 0 of a split row is
         // finished below)
-        const int nst = min(nr, kOutCap);
-        for (int r = lane; r < nst; r += 32)
-            if (!(r == 0 && need_lb)) out(y0 + r, s_out[r]);
+        constexpr int kAhead = RS::kAhead;
+        const int nst = min(nr, out_cap);
+        if constexpr (kAhead == 1) {
+            for (int r = lane; r < nst; r += 32)
+                if (!(r == 0 && need_lb)) out(y0 + r, *place(r));
+        } else {
+            for (int r0 = lane; r0 < nst; r0 += 32 * kAhead) {
+                int rr[kAhead];
+                double rows[kAhead];
+#pragma unroll
+                for (int q = 0; q < kAhead; ++q) {
+                    const int r = r0 + 32 * q;
+                    const bool mine = r < nst && !(r == 0 && need_lb);
+                    rr[q] = mine ? y0 + r : -1;
+                    rows[q] = mine ? *place(r) : 0.0;
+                }
+                out.rows(rr, rows);
+            }
+        }
 
         // ---- row y0 when it began in an earlier tile
         if (need_lb) {
@@ -415,7 +475,7 @@ struct WarpTile {
                     pb.carry = 0;
                 }
             } else {
-                if (nlb == kLookBackQueue) {  // warp-uniform
+                if (Src::kDrainInWalk && nlb == kLookBackQueue) {  // warp-uniform
                     drain_look_backs(src, epoch, lbq, nlb, lane, out);
                     nlb = 0;
                 }
@@ -424,7 +484,7 @@ struct WarpTile {
                     e.head = rv;
                     e.row = y0;
                     e.u = u;
-                    e.rs = rs;
+                    e.first = (int)((unsigned)(rs + y0) / (unsigned)(32 * IPT));
                     lbq[nlb] = e;
                 }
                 ++nlb;
