@@ -220,7 +220,7 @@ int merbit_spmm_dval(merbit_plan tplan, int32_t k, const void* d_g, int64_t ldg,
 
 /* Y[nrow x k] = alpha*A*X[ncol x k] + beta*Y, row-major with leading
  * dimensions ldx, ldy >= k (elements).  Any k >= 1 (processed in
- * power-of-two column blocks of at most 32).  The first call for a given
+ * column blocks of 32, the last one narrower).  The first call for a given
  * block width allocates that width's carry slots (synchronizes); later
  * calls allocate nothing and can be captured in a CUDA graph. */
 int merbit_spmm(merbit_plan plan, int32_t k, double alpha, const void* d_x, int64_t ldx,

@@ -78,8 +78,13 @@ SpmmDesc make_desc(merbit_plan_s* p, const Partition* part, const void* x, long 
     return d;
 }
 
-// One launch over columns [0, kk) of X / Y (pointers already offset).
-int spmm_block(merbit_plan_s* p, int kk, double alpha, const void* x, long long ldx, double beta,
+// No carry slots could be had for a kernel wider than the columns (under
+// capture, or out of memory): not a merbit_status.
+constexpr int kNoSlots = -1;
+
+// One launch over columns [0, cols) of X / Y (pointers already offset), by the
+// kernel of kk >= cols columns.
+int spmm_block(merbit_plan_s* p, int kk, int cols, double alpha, const void* x, long long ldx, double beta,
                void* y, long long ldy, cudaStream_t s, const void* dv_x = nullptr,
                long long dv_ldx = 0, void* dv_out = nullptr) {
     const int esz = (int)xy_size(p->dtype);
@@ -87,6 +92,7 @@ int spmm_block(merbit_plan_s* p, int kk, double alpha, const void* x, long long 
     // rows are loaded with the same width)
     auto width = [&](int items) {
         int vw = pick_vw(kk, ldx, x, y, ldy, esz, items);
+        while (vw > 1 && cols % vw != 0) vw >>= 1;  // a lane's columns are all used or none
         if (dv_out)
             while (vw > 1 && (dv_ldx % vw != 0 || (uintptr_t)dv_x % ((size_t)vw * esz) != 0)) vw >>= 1;
         return vw;
@@ -95,24 +101,28 @@ int spmm_block(merbit_plan_s* p, int kk, double alpha, const void* x, long long 
     // power-law and banded matrices, and among them the one of an odd length
     // per lane group (480, 496, 504, 508 items at k = 4, 8, 16, 32: no bank
     // conflicts between the groups' segments; Zipf-1M at k = 16: 0.524 ms
-    // against 0.570 at 512); other shapes keep 256
+    // against 0.570 at 512); two columns as one vector take the staged products
+    // of 352-item tiles (R-MAT-300k FP32: 59 us against 70 at 256; 87 before);
+    // other shapes keep 256
     int items = kDefaultItems;
     if (kk >= 4 && width(512) == 4) {
         items = 512;
         const int odd = spmm_odd_tile(kk);
         if (odd && width(odd) == 4) items = odd;
+    } else if (kk == 2 && !dv_out && width(352) == 2) {
+        items = 352;
     }
     const int vw = width(items);
     if (!spmm_config_exists(kk, vw, items)) return MERBIT_ERR_UNSUPPORTED;
     const Partition* part = nullptr;
     int st = plan_partition(p, items, &part, s);
-    if (st != MERBIT_OK) return st;
+    if (st != MERBIT_OK) return cols < kk ? kNoSlots : st;
     const long long key = ((long long)kk << 20) | items;
     auto it = p->spmm_slots.find(key);
     if (it == p->spmm_slots.end()) {
         SpmmSlots sl;
         st = alloc_spmm_slots(&sl, (long long)part->num_tiles * kk, s);
-        if (st != MERBIT_OK) return st;
+        if (st != MERBIT_OK) return cols < kk ? kNoSlots : st;
         it = p->spmm_slots.emplace(key, sl).first;
     }
     SpmmLaunch a = {};
@@ -124,6 +134,7 @@ int spmm_block(merbit_plan_s* p, int kk, double alpha, const void* x, long long 
     a.xch = it->second.words + 2 * (size_t)it->second.nslots;
     a.state = it->second.state;
     a.total_tiles = part->num_tiles;
+    a.cols = cols;
     a.alpha = alpha;
     a.beta = beta;
     if (dv_out) {
@@ -293,6 +304,7 @@ int batch_run(merbit_batch_s* b, double alpha, double beta, cudaStream_t s) {
     a.xch = b->slots.words + 2 * (size_t)b->slots.nslots;
     a.state = b->slots.state;
     a.total_tiles = b->total_tiles;
+    a.cols = b->k;
     a.alpha = alpha;
     a.beta = beta;
     if (b->kernel == 1) return batch_warp_launch(b->dtype, b->variant, a, s);
@@ -346,16 +358,25 @@ int merbit_spmm(merbit_plan plan, int32_t k, double alpha, const void* d_x, int6
     if (!d_y || (plan->ncol > 0 && !d_x)) return fail(MERBIT_ERR_INVALID, "spmm: X/Y is null");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t esz = xy_size(plan->dtype);
-    // power-of-two column blocks of at most 32
+    // Column blocks of 32; the rest in one launch of the smallest kernel that
+    // holds it, its lanes beyond the last column idle.  One launch per power of
+    // two read the matrix up to five times: R-MAT-300k (7.2 M nonzeros) FP32
+    // took 217, 512, 294 and 765 us at k = 12, 15, 20 and 31, and takes 113,
+    // 175, 153 and 252; no k from 2 to 40 is faster split.
     int j = 0;
     while (j < k) {
-        int kk = 32;
-        while (kk > k - j) kk >>= 1;
+        int cols = k - j < 32 ? k - j : 32;
+        int kk = 1;
+        while (kk < cols) kk <<= 1;
         const char* xb = static_cast<const char*>(d_x) + (size_t)j * esz;
         char* yb = static_cast<char*>(d_y) + (size_t)j * esz;
-        int st = spmm_block(plan, kk, alpha, xb, ldx, beta, yb, ldy, s);
+        int st = spmm_block(plan, kk, cols, alpha, xb, ldx, beta, yb, ldy, s);
+        if (st == kNoSlots) {  // as many columns as a narrower kernel's own
+            cols = kk = kk >> 1;
+            st = spmm_block(plan, kk, cols, alpha, xb, ldx, beta, yb, ldy, s);
+        }
         if (st != MERBIT_OK) return st;
-        j += kk;
+        j += cols;
     }
     return MERBIT_OK;
 }
@@ -373,7 +394,7 @@ int merbit_spmm_dval(merbit_plan tplan, int32_t k, const void* d_g, int64_t ldg,
     if (tplan->nrow == 0) return MERBIT_OK;
     if (!d_dx || !d_dval || (tplan->ncol > 0 && !d_g) || !d_x)
         return fail(MERBIT_ERR_INVALID, "spmm_dval: null pointer");
-    const int st = spmm_block(tplan, k, 1.0, d_g, ldg, 0.0, d_dx, lddx, (cudaStream_t)stream, d_x,
+    const int st = spmm_block(tplan, k, k, 1.0, d_g, ldg, 0.0, d_dx, lddx, (cudaStream_t)stream, d_x,
                               ldx, d_dval);
     if (st == MERBIT_ERR_UNSUPPORTED)
         return fail(MERBIT_ERR_UNSUPPORTED, "spmm_dval: no configuration for these operands");

@@ -613,6 +613,7 @@ struct SpmmLaunch {
     int nslots;
     LaunchState* state;
     int total_tiles;
+    int cols;  // right-hand sides: at most the kernel's K, a multiple of its vector width
     double alpha, beta;
     // Fused dL/dval (single matrix that is a transpose plan): for every
     // nonzero e of this matrix, dv_out[dv_perm[e]] = sum over the launch's

@@ -405,7 +405,7 @@ constexpr int kSpmmLookBacks = 8;
 template <int K, typename Y>
 __device__ __forceinline__ void spmm_look_back(const SpmmLookBack& e, unsigned long long* slots,
                                                unsigned long long* xch, LaunchState* st,
-                                               double alpha, double beta, int lane) {
+                                               double alpha, double beta, int cols, int lane) {
     constexpr int TPS = 32 / K;
     constexpr int R = 8;
     const int j = lane % K;
@@ -419,7 +419,7 @@ __device__ __forceinline__ void spmm_look_back(const SpmmLookBack& e, unsigned l
     __syncwarp();
 #pragma unroll
     for (int o = K; o < 32; o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    if (lane < K) {
+    if (lane < cols) {  // cols <= K
         const double head =
             __longlong_as_double((long long)ld_relaxed_u64(xch + (size_t)e.head * K + j));
         st_row(static_cast<Y*>(e.y), j, sum + head, alpha, beta);
@@ -433,7 +433,8 @@ __device__ __forceinline__ void drain_spmm_look_backs(const SpmmLookBack* q, int
     __syncwarp();
     const size_t par = (size_t)(epoch & 1u) * a.nslots;
     for (int i = 0; i < n; ++i)
-        spmm_look_back<K, Y>(q[i], a.slots + par, a.xch + par, a.state, a.alpha, a.beta, lane);
+        spmm_look_back<K, Y>(q[i], a.slots + par, a.xch + par, a.state, a.alpha, a.beta,
+                             a.cols, lane);
     __syncwarp();
 }
 
@@ -552,11 +553,14 @@ struct SpmmTile {
         const int g = lane / LPG;        // group
         const int jl = lane % LPG;       // lane within group
         const int j0 = jl * VW;          // first RHS column of this lane
+        // With fewer columns than K the lanes beyond them run along on the
+        // first lane's X (no further sectors) and store nothing.
+        const bool active = j0 < a.cols;
         // this lane's columns of X, and the distance of its rows in bytes (32
         // bits with vector loads: one wide multiply-add per address)
         using Step = typename std::conditional<(VW > 1), unsigned, unsigned long long>::type;
         const char* __restrict__ xl =
-            reinterpret_cast<const char*>(static_cast<const X*>(d.x) + j0);
+            reinterpret_cast<const char*>(static_cast<const X*>(d.x) + (active ? j0 : 0));
         const Step xstep = (Step)((unsigned long long)d.ldx * sizeof(X));
         char* __restrict__ yl = reinterpret_cast<char*>(static_cast<Y*>(d.y) + j0);
         const Step ystep = (Step)((unsigned long long)d.ldy * sizeof(Y));
@@ -572,6 +576,7 @@ struct SpmmTile {
                                      (VW * sizeof(Y) < 16 ? VW * sizeof(Y) - 1 : 15)) == 0;
         // row r of Y from its sum in double
         auto finish_row = [&](int r, const double (&v)[VW]) {
+            if (!active) return;
             Y* yr = y_row(r);
             if (plain) {
                 Y o[VW];
@@ -710,8 +715,8 @@ struct SpmmTile {
             } else if (plain) {
                 Y o[VW];
                 acc.rounded(o);
-                st_vec<VW>(y_row(y0 + ly), o, vecy);
-            } else {
+                if (active) st_vec<VW>(y_row(y0 + ly), o, vecy);
+            } else if (active) {
                 Y* yr = y_row(y0 + ly);
 #pragma unroll
                 for (int v = 0; v < VW; ++v) st_row(yr, v, acc.value(v), alpha, beta);
@@ -904,7 +909,7 @@ struct SpmmTile {
                 for (int v = 0; v < VW; ++v) {
                     st_relaxed_u64(xch + other + w + v, kEmpty);
                     const unsigned long long o = atomicExch(xch + par + w + v, dbits(sv[v]));
-                    if (o != kEmpty)
+                    if (o != kEmpty && active)
                         st_row(y_row(y1), v,
                                sv[v] + __longlong_as_double((long long)o), alpha, beta);
                 }
@@ -926,7 +931,7 @@ struct SpmmTile {
                     for (int v = 0; v < VW; ++v) {
                         const unsigned long long o =
                             atomicExch(xch + par + (size_t)u * K + j0 + v, dbits(rv[v]));
-                        if (o != kEmpty)
+                        if (o != kEmpty && active)
                             st_row(y_row(y0), v,
                                    __longlong_as_double((long long)o) + rv[v], alpha, beta);
                     }
@@ -974,12 +979,15 @@ struct SpmmStage {
 // registers).  On Zipf-1M FP32 at k = 16 the forward ran 427, 351 and 373 us
 // at 4, 5 and 6, and without a bound (80 registers, spills) 367.  FP64 with the
 // fused dval, with two tile sizes or with 8 scalar gathers ahead would spill
-// at 5.
-template <int DT, int VW, int ITEMS2, bool DV>
-constexpr int kSpmmMinCtas = DT == MERBIT_F64 && (DV || ITEMS2 != 0 || VW == 1) ? 4 : 5;
+// at 5; FP32 with staged products takes 6 (80 registers; an 80 x 70 x 60
+// 27-point stencil at k = 2: 80, 71, 68 and 76 us at 4, 5, 6 and 7).
+template <int DT, int K, int VW, int ITEMS, int ITEMS2, bool DV>
+constexpr int kSpmmMinCtas =
+    DT == MERBIT_F64 ? (DV || ITEMS2 != 0 || VW == 1 ? 4 : 5)
+                     : (SpmmTile<DT, K, VW, ITEMS, DV>::STAGEP ? 6 : 5);
 
 template <int DT, int K, int VW, int ITEMS, int ITEMS2, int WARPS, bool DV>
-__global__ void __launch_bounds__(WARPS * 32, kSpmmMinCtas<DT, VW, ITEMS2, DV>)
+__global__ void __launch_bounds__(WARPS * 32, kSpmmMinCtas<DT, K, VW, ITEMS, ITEMS2, DV>)
     spmm_kernel(const SpmmLaunch a) {
     using St = SpmmStage<DT, K, VW, ITEMS, ITEMS2, DV>;
     using T = typename St::T1;

@@ -67,6 +67,58 @@ def test_rows_at_segment_and_tile_ends(dtype, k, alpha, beta, pad):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("k", [1, 2, 3, 5, 6, 7, 9, 12, 15, 17, 18, 20, 24, 28, 31, 33, 44])
+@pytest.mark.parametrize("dtype,pad", [("f32", 0), ("f32", 4), ("f64", 2), ("bf16", 1)])
+def test_columns_that_are_no_power_of_two(dtype, pad, k):
+    """A launch whose last lanes have no column: every vector width that k and
+    the leading dimension give, rows over several tiles among them, and the
+    columns of X and Y beyond k neither read into the result nor written."""
+    A = _matrix(16, seed=2)
+    xy = np.float64 if dtype == "f64" else np.float32
+    X = synth.uniform(11, A.ncol * (k + pad)).reshape(A.ncol, k + pad).astype(xy)
+    X[:, k:] = np.nan
+    Y0 = synth.uniform(12, A.nrow * (k + pad)).reshape(A.nrow, k + pad).astype(xy)
+    plan = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
+    yo, ya = O.spmm(A.row_ptr, A.col, stored_values(A, dtype), X[:, :k].copy(), k=k)
+    yo, ya = yo.reshape(-1, k), ya.reshape(-1, k)
+    for alpha, beta in ((1.0, 0.0), (2.0, 0.5)):
+        Yd = torch.from_numpy(Y0).cuda()
+        plan.spmm(torch.from_numpy(X).cuda()[:, :k], Yd[:, :k], alpha=alpha, beta=beta)
+        got = Yd.cpu().numpy()
+        want = alpha * yo + beta * Y0[:, :k].astype(np.float64)
+        scale = abs(alpha) * ya + abs(beta) * np.abs(Y0[:, :k])
+        assert (np.abs(got[:, :k] - want) <= TOL[dtype] * np.maximum(scale, 1e-300)).all()
+        assert np.array_equal(got[:, k:], Y0[:, k:])
+    plan.check()
+
+
+@pytest.mark.gpu
+def test_captured_product_with_the_slots_of_narrower_ones():
+    """A product of 20 columns captured after products of 16 and 4 (whose
+    carry slots the plan then holds), as when each power of two had its own."""
+    A = _matrix(16, seed=3)
+    k = 20
+    X = synth.uniform(13, A.ncol * k).reshape(A.ncol, k).astype(np.float32)
+    plan = mb.Plan(*to_cuda(A, "f32"), ncol=A.ncol)
+    xd = torch.from_numpy(X).cuda()
+    Yd = torch.zeros(A.nrow, k, dtype=torch.float32, device="cuda")
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        plan.spmm(xd[:, :16], Yd[:, :16])
+        plan.spmm(xd[:, 16:], Yd[:, 16:])
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        plan.spmm(xd, Yd, stream=s)
+    yo, ya = O.spmm(A.row_ptr, A.col, A.vals.astype(np.float32), X, k=k)
+    for _ in range(3):
+        Yd.fill_(float("nan"))
+        g.replay()
+        torch.cuda.synchronize()
+        assert (np.abs(Yd.cpu().numpy() - yo) <= 1e-6 * np.maximum(ya, 1e-300)).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["f64", "f32"])
 @pytest.mark.parametrize("k", [1, 2, 4, 8, 16, 32])
 def test_fused_backward_at_segment_and_tile_ends(dtype, k):
