@@ -122,10 +122,47 @@ int plan_config_ok(merbit_plan_s* p, int idx, bool* ok, cudaStream_t s) {
     return MERBIT_OK;
 }
 
-// First usable configuration in table order.
+// The untuned choice for a matrix whose longest row is short: row groups, -1
+// for the merge-path kernels.  Measured on B200 against the merge-path default
+// (us; FP64 / FP32; longest row, mean):
+//   27-point stencil 160^3 (27, 26.7)      250 / 177   against 503 / 411
+//   5-point Laplacian 2048^2 (5, 5)        108 /  64   against 111 /  96
+//   random rows of 3 and of 12             91 / 78 and 63 / 54   against 98 / 92, 89 / 74
+//   random rows of 28, of 64, of 0 to 100  101 / 91, 118 / 113, 105 / 98
+//                                          against 131 / 109, 163 / 128, 127 / 103
+//   random rows of 2                       56 / 50   against 55 / 45 (not taken)
+// Short rows (mean below 14, none above 32) go one per lane through shared
+// memory, longer ones to 4 lanes, from a mean of 40 to 8: rows of 12 take 63
+// us at one lane and 65 at 4, of 16 135 and 90; of 32 95 at 4 lanes and 93 at 8, of
+// 64 85 and 72 (FP64).  Above 128 entries a row the rule leaves the matrix to
+// the merge path, which balances any rows.
+constexpr int kShortRows = 128;
+int short_rows_choice(const merbit_plan_s* p) {
+    if (p->max_row_len < 1 || p->max_row_len > kShortRows) return -1;
+    const double mean = (double)p->nnz / (double)std::max(p->nrow, 1);
+    if (mean < 2.5) return -1;
+    const bool lane_per_row = mean < 14.0 && p->max_row_len <= 32;
+    const int lanes = lane_per_row ? 1 : mean < 40.0 ? 4 : 8;
+    for (int i = 0, n = spmv_num_configs(p->dtype); i < n; ++i) {
+        const SpmvConfig c = spmv_config(p->dtype, i);
+        if (c.kind == 3 && c.ipt == lanes && !c.cg && (c.stg != 0) == lane_per_row) return i;
+    }
+    return -1;
+}
+
+// First usable configuration in table order; when the tiles of the first end
+// more rows than its row_ptr window holds (runs of empty and one-entry rows, as
+// in R-MAT graphs), the first whose window holds a tile of row ends.
 int plan_pick_default(merbit_plan_s* p, cudaStream_t s) {
     const int n = spmv_num_configs(p->dtype);
-    for (int i = 0; i < n; ++i) {
+    std::vector<int> order;
+    for (int pass = 0; pass < 2; ++pass)
+        for (int i = 0; i < n; ++i) {
+            const SpmvConfig c = spmv_config(p->dtype, i);
+            const bool early = i == 0 || (c.kind == 1 && c.stg);
+            if (early == (pass == 0)) order.push_back(i);
+        }
+    for (int i : order) {
         bool ok = false;
         int st = plan_config_ok(p, i, &ok, s);
         if (st != MERBIT_OK) return st;
@@ -394,9 +431,13 @@ int merbit_plan_create(merbit_plan* plan, int32_t nrow, int32_t ncol, int32_t nn
                 tuned = it->second.cfg;
         }
         bool ok = false;
+        const int rule = tuned < 0 ? short_rows_choice(p) : -1;
         if (tuned >= 0) {
             st = plan_config_ok(p, tuned, &ok, s);  // reuses the partition built above
             if (st == MERBIT_OK && ok) p->cfg = tuned;
+        } else if (rule >= 0) {
+            p->cfg = rule;  // row groups take any matrix
+            ok = true;
         } else {
             // no cached choice for this signature: the provisional one came
             // from another longest-row bucket, so it is not kept
