@@ -3,12 +3,16 @@
 //
 //   merbit_coo_sort        GRAPH::sort (src/class.cu:143-177): order the COO
 //                          triplets by (major, minor); a stable radix sort
-//                          of the 64-bit key major<<32|minor, then a gather
+//                          of one 64-bit word per triplet that holds major,
+//                          minor and the triplet's position, over the bits
+//                          that major and minor use, then a gather
 //   merbit_coo_to_csr      cusparseXcoo2csr (include/tile.cuh:574): offsets
 //                          of a sorted index array
 //   merbit_outdegree_values Fun_Values (src/class.cu:2-34): value = 1 /
 //                          (number of entries whose row_ind equals this
 //                          entry's row_ind)
+#include <algorithm>
+
 #include <cub/device/device_radix_sort.cuh>
 
 #include "merbit_internal.cuh"
@@ -36,6 +40,49 @@ __global__ void unpack_keys(const unsigned long long* __restrict__ key, int n,
         major[i] = (int)(key[i] >> 32);
         minor[i] = (int)(key[i] & 0xFFFFFFFFull);
     }
+}
+
+// Largest index of each array, as unsigned values.
+__global__ void max_indices(const int* __restrict__ major, const int* __restrict__ minor, int n,
+                            unsigned* __restrict__ out) {
+    unsigned a = 0u, b = 0u;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        a = max(a, (unsigned)major[i]);
+        b = max(b, (unsigned)minor[i]);
+    }
+    a = __reduce_max_sync(0xFFFFFFFFu, a);
+    b = __reduce_max_sync(0xFFFFFFFFu, b);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(out, a);
+        atomicMax(out + 1, b);
+    }
+}
+
+// One word per triplet: major, minor (b_minor bits) and position (b_pos bits).
+__global__ void pack_words(const int* __restrict__ major, const int* __restrict__ minor, int n,
+                           int b_minor, int b_pos, unsigned long long* __restrict__ word) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        word[i] = ((((unsigned long long)(unsigned)major[i] << b_minor) | (unsigned)minor[i]) << b_pos) |
+                  (unsigned)i;
+}
+
+template <typename V>
+__global__ void unpack_words(const unsigned long long* __restrict__ word, int n, int b_minor,
+                             int b_pos, int* __restrict__ major, int* __restrict__ minor,
+                             const V* __restrict__ src, V* __restrict__ dst) {
+    const unsigned long long pos = (1ull << b_pos) - 1, min_mask = (1ull << b_minor) - 1;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned long long w = word[i];
+        major[i] = (int)(w >> (b_minor + b_pos));
+        minor[i] = (int)((w >> b_pos) & min_mask);
+        if (src) dst[i] = src[w & pos];
+    }
+}
+
+int bits_of(unsigned long long v) {
+    int b = 0;
+    while (v >> b) ++b;
+    return b;
 }
 
 template <typename V>
@@ -109,8 +156,49 @@ int merbit_coo_sort(int32_t nnz, int32_t* d_major, int32_t* d_minor, void* d_val
         int _st = dev_alloc(&(p), (bytes), s);           \
         if (_st != MERBIT_OK) return done(_st);          \
     } while (0)
+    // Indices of b1 and b2 bits and positions of b3 fit one word as a rule: then
+    // keys alone are sorted, over b1 + b2 bits, between two buffers, and the
+    // buffer that is free afterwards takes the values.  4 M triplets of a 250,000
+    // node graph: 5 passes over 8 bytes instead of 8 over 12 (0.19 ms instead of
+    // 0.42), and 64 MB of work space instead of 180, which the pool can keep
+    // (it unmapped the rest at every call: 2 to 13 ms).
     TRY_ALLOC(k_in, 8 * (size_t)nnz);
     TRY_ALLOC(k_out, 8 * (size_t)nnz);
+    unsigned top[2] = {0u, 0u};
+    unsigned* d_top = reinterpret_cast<unsigned*>(k_out);  // not in use yet
+    TRY(cudaMemsetAsync(d_top, 0, sizeof(top), s));
+    max_indices<<<grid_of(nnz), 256, 0, s>>>(d_major, d_minor, nnz, d_top);
+    TRY(cudaMemcpyAsync(top, d_top, sizeof(top), cudaMemcpyDeviceToHost, s));
+    TRY(cudaStreamSynchronize(s));
+    const int b_pos = bits_of((unsigned)(nnz - 1));
+    const int b_minor = std::max(bits_of(top[1]), 1);
+    const int b_all = b_pos + b_minor + std::max(bits_of(top[0]), 1);
+    if (b_all <= 64) {
+        pack_words<<<grid_of(nnz), 256, 0, s>>>(d_major, d_minor, nnz, b_minor, b_pos, k_in);
+        cub::DoubleBuffer<unsigned long long> words(k_in, k_out);
+        size_t tb = 0;
+        TRY(cub::DeviceRadixSort::SortKeys(nullptr, tb, words, nnz, b_pos, b_all, s));
+        TRY_ALLOC(temp, tb);
+        TRY(cub::DeviceRadixSort::SortKeys(temp, tb, words, nnz, b_pos, b_all, s));
+        if (d_vals)
+            TRY(cudaMemcpyAsync(words.Alternate(), d_vals, vs * (size_t)nnz,
+                                cudaMemcpyDeviceToDevice, s));
+#define UNPACK(V)                                                                             \
+    unpack_words<V><<<grid_of(nnz), 256, 0, s>>>(                                             \
+        words.Current(), nnz, b_minor, b_pos, d_major, d_minor,                               \
+        d_vals ? reinterpret_cast<const V*>(words.Alternate()) : nullptr, static_cast<V*>(d_vals))
+        if (dtype == MERBIT_F64)
+            UNPACK(double);
+        else if (dtype == MERBIT_F32)
+            UNPACK(float);
+        else
+            UNPACK(unsigned short);
+#undef UNPACK
+        TRY(cudaGetLastError());
+        TRY(cudaStreamSynchronize(s));
+        return done(MERBIT_OK);
+    }
+    // wider indices (or negative ones, as unsigned): 64-bit keys and positions
     TRY_ALLOC(i_in, 4 * (size_t)nnz);
     TRY_ALLOC(i_out, 4 * (size_t)nnz);
     pack_keys<<<grid_of(nnz), 256, 0, s>>>(d_major, d_minor, nnz, k_in, i_in);
