@@ -27,7 +27,7 @@
 // slots that a launch uses are emptied for the next one (all of them, they
 // were 20 MB of L2 for Zipf-1M at k = 16, whose X of 64 MB then no longer fit).
 // Measured on B200, before and after: Zipf-1M FP32 k = 16 526 -> 351 us, its
-// fused backward 628 -> 550; Zipf-500k FP64 k = 8 210 -> 153; 32 R-MAT
+// fused backward 628 -> 537; Zipf-500k FP64 k = 8 210 -> 153; 32 R-MAT
 // matrices FP32 in one launch, k = 4 603 -> 435, k = 32 1,540 -> 1,070.
 //
 // Batches: the tiles of all matrices form one index space; matrix m owns
@@ -650,61 +650,33 @@ struct SpmmTile {
         }
         next_row(lx);
 
-        // fused dval: this lane's VW values of dv_x's current row, and of the
-        // row after it (loaded one row ahead: a row start would otherwise
-        // wait for its load)
+        // fused dval: this lane's VW values of dv_x's current row.  (Loading
+        // the row after it ahead, or one shuffle tree for two nonzeros, was no
+        // faster: Zipf-1M FP32 at k = 16 took 542 and 539 us against 537.  The
+        // scattered dval writes bind this form: their 97 MB and G's 64 MB
+        // do not fit L2 together.)
         const int* perm_t = reinterpret_cast<const int*>(ws + perm_offset) - (x0 & ~3);
-        XRow<X, VW> xrow, xnext;
-        int xnext_of = 0;
-        auto dv_load = [&](int r, XRow<X, VW>& o) {
-            if (r <= ly_end && y0 + r < nrow)
-                o.load(static_cast<const X*>(a.dv_x) + (size_t)(y0 + r) * a.dv_ldx + j0);
-        };
-        auto dv_next = [&]() {  // ly is the current row
-            if (xnext_of == ly)
-                xrow = xnext;
-            else
-                dv_load(ly, xrow);
-            xnext_of = ly + 1;
-            dv_load(xnext_of, xnext);
+        XRow<X, VW> xrow;
+        auto dv_row = [&]() {  // ly is the current row
+            if (y0 + ly < nrow)
+                xrow.load(static_cast<const X*>(a.dv_x) + (size_t)(y0 + ly) * a.dv_ldx + j0);
         };
         if (DV) {
             xrow.zero();
-            xnext.zero();
-            xnext_of = -1;
-            dv_next();
+            dv_row();
         }
         const unsigned gmask = LPG == 32 ? 0xFFFFFFFFu : (((1u << LPG) - 1u) << (g * LPG));
-        // dval of nonzero e (and e + 1 of the same row): in the x type, VW
-        // fused multiply-adds per lane, then a tree over the group's lanes
-        // (error within (VW + log2 LPG) roundings of sum |g x|)
-        auto dv_dot = [&](const XRow<X, VW>& xr) {
+        // dval of nonzero e: in the x type, VW fused multiply-adds per lane, then
+        // a tree over the group's lanes (error within (VW + log2 LPG) roundings
+        // of sum |g x|)
+        X* __restrict__ dvo = static_cast<X*>(a.dv_out);
+        auto dv_one = [&](int e, const XRow<X, VW>& xr) {
             X dd = (X)0;
 #pragma unroll
             for (int v = 0; v < VW; ++v) dd = fma(xr[v], xrow[v], dd);
-            return dd;
-        };
-        X* __restrict__ dvo = static_cast<X*>(a.dv_out);
-        auto dv_one = [&](int e, const XRow<X, VW>& xr) {
-            X dd = dv_dot(xr);
 #pragma unroll
-            for (int o = 1; o < LPG; o <<= 1) dd += __shfl_xor_sync(gmask, dd, o);
+            for (int o = LPG / 2; o > 0; o >>= 1) dd += __shfl_xor_sync(gmask, dd, o);
             if (jl == 0) dvo[perm_t[e]] = dd;
-        };
-        auto dv_two = [&](int e, const XRow<X, VW>& xr0, const XRow<X, VW>& xr1) {
-            const X d0 = dv_dot(xr0), d1 = dv_dot(xr1);
-            if (LPG == 1) {
-                dvo[perm_t[e]] = d0;
-                dvo[perm_t[e + 1]] = d1;
-            } else {
-                // even lanes sum the first, odd lanes the second: one exchange
-                // halves the two trees into one
-                const bool odd = (jl & 1) != 0;
-                X dd = (odd ? d1 : d0) + __shfl_xor_sync(gmask, odd ? d0 : d1, 1);
-#pragma unroll
-                for (int o = 2; o < LPG; o <<= 1) dd += __shfl_xor_sync(gmask, dd, o);
-                if (jl < 2) dvo[perm_t[e + jl]] = dd;
-            }
         };
 
         // the current row ends at nonzero e
@@ -724,7 +696,7 @@ struct SpmmTile {
             acc.zero();
             ++ly;
             next_row(e);
-            if (DV) dv_next();
+            if (DV) dv_row();
         };
 
         // ---- walk: chunks of CH nonzeros, the next chunk's x rows in flight
@@ -751,7 +723,10 @@ struct SpmmTile {
                 if constexpr (CH == 2) {
                     // F32/BF16: one compensated addition of the fused pair
                     acc.add_two(to_p(vv[0]), xr[0], to_p(vv[1]), xr[1]);
-                    if (DV) dv_two(c, xr[0], xr[1]);
+                    if (DV) {
+                        dv_one(c, xr[0]);
+                        dv_one(c + 1, xr[1]);
+                    }
                 } else {
 #pragma unroll
                     for (int t = 0; t < CH; ++t) {
@@ -766,10 +741,8 @@ struct SpmmTile {
                 if (c < lx_end) {
                     acc.add_two(to_p(vv[0]), xr[0], to_p(vv[1]), xr[1], both);
                     if (DV) {
-                        if (both)
-                            dv_two(c, xr[0], xr[1]);
-                        else
-                            dv_one(c, xr[0]);
+                        dv_one(c, xr[0]);
+                        if (both) dv_one(c + 1, xr[1]);
                     }
                     if (next_end == c + 1) {
                         end_row(c + 1);
