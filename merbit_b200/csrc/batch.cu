@@ -112,8 +112,19 @@ int spmm_block(merbit_plan_s* p, int kk, int cols, double alpha, const void* x, 
     } else if (kk == 2 && !dv_out && width(352) == 2) {
         items = 352;
     }
-    const int vw = width(items);
+    int vw = width(items);
     if (!spmm_config_exists(kk, vw, items)) return MERBIT_ERR_UNSUPPORTED;
+    // Vector width 2 in tiles of an odd length per lane group: where the operands
+    // allow no more (FP32 k = 6: 95 us against 109 in 256-item tiles; R-MAT-300k),
+    // and in FP64, whose 16-byte loads then take a lane's whole slice and half
+    // as many groups diverge at row ends: k = 4 76 us against 88, k = 32 181
+    // against 190; on an 80 x 70 x 60 27-point stencil k = 8 98 against 120, k = 32
+    // 209 against 250; on Zipf-300k k = 32 227 against 301.  Not at 9 to 16 columns:
+    // k = 16 on Zipf-300k takes 152 us against 129.
+    if (!dv_out && kk >= 4 && (vw == 2 || (vw == 4 && p->dtype == MERBIT_F64 && kk != 16))) {
+        items = spmm_odd_tile2(kk);
+        vw = 2;
+    }
     const Partition* part = nullptr;
     int st = plan_partition(p, items, &part, s);
     if (st != MERBIT_OK) return cols < kk ? kNoSlots : st;

@@ -667,6 +667,9 @@ bool spmm_config_exists(int k, int vw, int items);
 // length per lane group at vector width 4 (0 if k has none).
 int spmm_tile_candidates(int k, int* out);
 int spmm_odd_tile(int k);
+// The tile of an odd length per lane group at vector width 2, which single
+// matrices take (not among the batch's candidates; 0 if k has none).
+int spmm_odd_tile2(int k);
 
 }  // namespace merbit
 

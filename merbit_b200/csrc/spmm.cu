@@ -1125,6 +1125,15 @@ int launch_spmm_dt(int k, int vw, int items, int items2, const SpmmLaunch& a, cu
     MERBIT_SPMM_CASE(2, 2, 224)
     MERBIT_SPMM_CASE(2, 2, 352)
 #undef MERBIT_SPMM_CASE
+    // odd segments at vector width 2 (single matrices without the fused dval)
+#define MERBIT_SPMM_PLAIN_CASE(KK, VV, II)                  \
+    if (k == KK && vw == VV && items == II && !a.dv_out)    \
+        return launch_spmm_cfg<DT, KK, VV, II, 4, false>(a, s);
+    MERBIT_SPMM_PLAIN_CASE(4, 2, 496)
+    MERBIT_SPMM_PLAIN_CASE(8, 2, 504)
+    MERBIT_SPMM_PLAIN_CASE(16, 2, 508)
+    MERBIT_SPMM_PLAIN_CASE(32, 2, 510)
+#undef MERBIT_SPMM_PLAIN_CASE
     return fail(MERBIT_ERR_INVALID, "spmm: no such configuration");
 }
 
@@ -1166,6 +1175,16 @@ int spmm_odd_tile(int k) {
     case 8: return 496;
     case 16: return 504;
     case 32: return 508;
+    }
+    return 0;
+}
+
+int spmm_odd_tile2(int k) {
+    switch (k) {
+    case 4: return 496;
+    case 8: return 504;
+    case 16: return 508;
+    case 32: return 510;
     }
     return 0;
 }

@@ -19,10 +19,13 @@ TOL = {"f64": 1e-13, "f32": 1e-6, "bf16": 1e-6}
 # merge items of a lane group's segment and of a tile (vector width 4)
 SEG = {4: 15, 8: 31, 16: 63, 32: 127}
 TILE = {4: 480, 8: 496, 16: 504, 32: 508}
+# and at vector width 2 (FP64, and widths that are no multiple of 4)
+SEG2 = {4: 31, 8: 63, 16: 127, 32: 255}
+TILE2 = {4: 496, 8: 504, 16: 508, 32: 510}
 
 
-def _lengths(k):
-    s, t = SEG[k], TILE[k]
+def _lengths(k, seg=SEG, tile=TILE):
+    s, t = seg[k], tile[k]
     rng = np.random.default_rng(k)
     return np.concatenate([
         np.arange(s - 3, s + 3).repeat(9),           # row ends drift over segment ends
@@ -34,8 +37,9 @@ def _lengths(k):
     ]).astype(np.int64)
 
 
-def _matrix(k, seed=0):
-    return csr_from_lengths(_lengths(k), ncol=4000, seed=seed)
+def _matrix(k, seed=0, width2=False):
+    L = _lengths(k, SEG2, TILE2) if width2 else _lengths(k)
+    return csr_from_lengths(L, ncol=4000, seed=seed)
 
 
 @pytest.mark.gpu
@@ -90,6 +94,31 @@ def test_columns_that_are_no_power_of_two(dtype, pad, k):
         assert (np.abs(got[:, :k] - want) <= TOL[dtype] * np.maximum(scale, 1e-300)).all()
         assert np.array_equal(got[:, k:], Y0[:, k:])
     plan.check()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["f64", "f32", "bf16"])
+@pytest.mark.parametrize("kk", [4, 8, 16, 32])
+@pytest.mark.parametrize("alpha,beta", [(1.0, 0.0), (-0.5, 2.0)])
+def test_vector_width_two_at_segment_and_tile_ends(dtype, kk, alpha, beta):
+    """k = kk - 2 (and kk in FP64): tiles of an odd length per group of kk/2 lanes."""
+    A = _matrix(kk, seed=4, width2=True)
+    xy = np.float64 if dtype == "f64" else np.float32
+    for k in ([kk - 2, kk] if dtype == "f64" else [kk - 2]):
+        if k < 3:
+            continue
+        X = synth.uniform(15, A.ncol * k).reshape(A.ncol, k).astype(xy)
+        Y0 = synth.uniform(16, A.nrow * k).reshape(A.nrow, k).astype(xy)
+        plan = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
+        yo, ya = O.spmm(A.row_ptr, A.col, stored_values(A, dtype), X, k=k)
+        want = alpha * yo + beta * Y0.astype(np.float64)
+        scale = abs(alpha) * ya + abs(beta) * np.abs(Y0)
+        for _ in range(2):  # either slot parity
+            Yd = torch.from_numpy(Y0).cuda()
+            plan.spmm(torch.from_numpy(X).cuda(), Yd, alpha=alpha, beta=beta)
+            got = Yd.cpu().numpy()
+            assert (np.abs(got - want) <= TOL[dtype] * np.maximum(scale, 1e-300)).all()
+        plan.check()
 
 
 @pytest.mark.gpu
