@@ -78,6 +78,31 @@ SpmmDesc make_desc(merbit_plan_s* p, const Partition* part, const void* x, long 
     return d;
 }
 
+// Warps of the SpMM kernel that the device holds: 5 CTAs of 4 per SM.
+int spmm_warps() {
+    static int sms[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return 148 * 20;
+    int n = __atomic_load_n(&sms[dev], __ATOMIC_RELAXED);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
+        __atomic_store_n(&sms[dev], n, __ATOMIC_RELAXED);
+    }
+    return 20 * n;
+}
+
+// What a launch with tiles of `items` merge items takes, in items: the rounds
+// of its busiest warp, each tile costing about kTileCost items beyond its own.
+constexpr int kTileCost = 100;
+long long tile_rounds(const merbit_plan_s* p, int items, int warps) {
+    const long long tiles = ((long long)p->nrow + p->nnz + items - 1) / items;
+    return (tiles + warps - 1) / warps;
+}
+long long tile_cost(const merbit_plan_s* p, int items, int warps) {
+    return tile_rounds(p, items, warps) * (items + kTileCost);
+}
+
 // No carry slots could be had for a kernel wider than the columns (under
 // capture, or out of memory): not a merbit_status.
 constexpr int kNoSlots = -1;
@@ -124,6 +149,19 @@ int spmm_block(merbit_plan_s* p, int kk, int cols, double alpha, const void* x, 
     if (!dv_out && kk >= 4 && (vw == 2 || (vw == 4 && p->dtype == MERBIT_F64 && kk != 16))) {
         items = spmm_odd_tile2(kk);
         vw = 2;
+    }
+    // Small matrices: the larger tile leaves warps without one, or most of a last
+    // round without work.  Up to 8 columns the smaller tile is taken when it fills
+    // one round at most (beyond, its overhead was seen to cost up to 15%), for more
+    // columns whenever its rounds cost less.  R-MAT of degree 30, us, larger / smaller
+    // tile: 2,000 rows FP32 k = 4, 16, 32 13 / 12, 22 / 16, 32 / 20; 20,000 rows FP64
+    // k = 8 28 / 21; 60,000 rows FP32 k = 32 58 / 51.
+    const int small = vw == 4 ? spmm_small_tile(kk) : vw == 2 ? kDefaultItems : items;
+    if (kk >= 4 && small < items && spmm_config_exists(kk, vw, small)) {
+        const int warps = spmm_warps();
+        const bool one_round = tile_rounds(p, small, warps) <= 1;
+        if ((kk >= 16 || one_round) && tile_cost(p, small, warps) < tile_cost(p, items, warps))
+            items = small;
     }
     const Partition* part = nullptr;
     int st = plan_partition(p, items, &part, s);

@@ -167,33 +167,14 @@ __device__ __forceinline__ void publish_carry(unsigned long long* slots, int nsl
     st_relaxed_u64(slots + (size_t)(epoch & 1u) * nslots + t, b);
 }
 
-// Reads tile t's carry, waiting (bounded) until it is published.
-__device__ __forceinline__ double read_carry(const unsigned long long* slots, int nslots,
-                                             unsigned epoch, int t, LaunchState* st,
-                                             unsigned long long wait_ns = kCarryWaitNs) {
-    const unsigned long long* p = slots + (size_t)(epoch & 1u) * nslots + t;
-    unsigned long long b = ld_relaxed_u64(p);
-    if (b != kEmpty) return __longlong_as_double((long long)b);
-    const unsigned long long t0 = global_timer_ns();
-    for (;;) {
-        __nanosleep(32);
-        b = ld_relaxed_u64(p);
-        if (b != kEmpty) return __longlong_as_double((long long)b);
-        if (*(volatile int*)&st->error != 0) return 0.0;
-        if (global_timer_ns() - t0 > wait_ns) {
-            atomicExch(&st->error, (int)MERBIT_ERR_TIMEOUT);
-            return 0.0;
-        }
-    }
-}
-
 // Loads the carries p[0], p[stride], ... (those at offsets below `left`; +0.0
 // for the others), all in flight together, waiting (bounded) until each is
 // published.
 template <int N>
 __device__ __forceinline__ void load_carries(unsigned long long (&b)[N],
                                              const unsigned long long* p, int stride, int left,
-                                             LaunchState* st) {
+                                             LaunchState* st,
+                                             unsigned long long wait_ns = kCarryWaitNs) {
     bool missing = false;
 #pragma unroll
     for (int r = 0; r < N; ++r) {
@@ -211,7 +192,7 @@ __device__ __forceinline__ void load_carries(unsigned long long (&b)[N],
             missing = missing || b[r] == kEmpty;
         }
         if (!missing) return;
-        const bool late = global_timer_ns() - t0 > kCarryWaitNs;
+        const bool late = global_timer_ns() - t0 > wait_ns;
         if (late) atomicExch(&st->error, (int)MERBIT_ERR_TIMEOUT);
         if (late || *(volatile int*)&st->error != 0) break;
     }
@@ -667,6 +648,7 @@ bool spmm_config_exists(int k, int vw, int items);
 // length per lane group at vector width 4 (0 if k has none).
 int spmm_tile_candidates(int k, int* out);
 int spmm_odd_tile(int k);
+int spmm_small_tile(int k);  // the smaller of the two odd tiles
 // The tile of an odd length per lane group at vector width 2, which single
 // matrices take (not among the batch's candidates; 0 if k has none).
 int spmm_odd_tile2(int k);

@@ -12,8 +12,8 @@ __device__ unsigned long long g_never_published = kEmpty;
 
 __global__ void carry_wait_kernel(LaunchState* st, unsigned long long wait_ns) {
     if (threadIdx.x != 0) return;
-    // nslots = 0: both parities resolve to the same never-published word
-    (void)read_carry(&g_never_published, 0, 0u, 0, st, wait_ns);
+    unsigned long long b[1];
+    load_carries<1>(b, &g_never_published, 1, 1, st, wait_ns);
 }
 
 __global__ void mbar_wait_kernel(LaunchState* st, unsigned long long wait_ns) {

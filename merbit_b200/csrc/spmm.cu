@@ -1179,6 +1179,16 @@ int spmm_odd_tile(int k) {
     return 0;
 }
 
+int spmm_small_tile(int k) {
+    switch (k) {
+    case 4: return 288;
+    case 8: return 272;
+    case 16: return 264;
+    case 32: return 260;
+    }
+    return 0;
+}
+
 int spmm_odd_tile2(int k) {
     switch (k) {
     case 4: return 496;
@@ -1192,7 +1202,7 @@ int spmm_odd_tile2(int k) {
 bool spmm_pair_exists(int k, int vw, int items, int items2) {
     if (vw != 4 || !(k == 4 || k == 8 || k == 16 || k == 32)) return false;
     if (items == 256 && items2 == 512) return true;
-    return items2 == spmm_odd_tile(k) && items == (k == 4 ? 288 : k == 8 ? 272 : k == 16 ? 264 : 260);
+    return items2 == spmm_odd_tile(k) && items == spmm_small_tile(k);
 }
 
 int spmm_launch(int dtype, int k, int vw, int items, const SpmmLaunch& a, cudaStream_t s,

@@ -122,6 +122,31 @@ def test_vector_width_two_at_segment_and_tile_ends(dtype, kk, alpha, beta):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("k", [4, 8, 16, 32])
+def test_tiles_of_small_and_large_matrices_agree_with_the_oracle(dtype, k):
+    """Matrices on both sides of one round of the smaller tile, long rows in
+    them: whichever tile the size picks gives the oracle's product."""
+    xy = np.float64 if dtype == "f64" else np.float32
+    rng = np.random.default_rng(k)
+    for rows in (300, 18_000, 24_000, 40_000):
+        L = rng.integers(0, 60, rows)
+        L[rows // 2] = 3000
+        rp = np.zeros(rows + 1, np.int32)
+        np.cumsum(L, out=rp[1:])
+        nnz = int(rp[-1])
+        A = synth.CSR(rp, rng.integers(0, 5000, nnz, dtype=np.int32), rng.standard_normal(nnz), 5000)
+        X = synth.uniform(17, A.ncol * k).reshape(A.ncol, k).astype(xy)
+        plan = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
+        yo, ya = O.spmm(A.row_ptr, A.col, stored_values(A, dtype), X, k=k)
+        xd = torch.from_numpy(X).cuda()
+        for _ in range(2):
+            Y = plan.spmm(xd).cpu().numpy()
+            assert (np.abs(Y - yo) <= TOL[dtype] * np.maximum(ya, 1e-300)).all()
+        plan.check()
+
+
+@pytest.mark.gpu
 def test_captured_product_with_the_slots_of_narrower_ones():
     """A product of 20 columns captured after products of 16 and 4 (whose
     carry slots the plan then holds), as when each power of two had its own."""
