@@ -152,7 +152,9 @@ int merbit_plan_set_config(merbit_plan plan, int32_t idx, void* stream);
 /* *usable = 1 when configuration idx can run this plan (same rules). */
 int merbit_plan_config_usable(merbit_plan plan, int32_t idx, int32_t* usable, void* stream);
 
-/* y[nrow] = alpha*A*x[ncol] + beta*y.  beta == 0 never reads y. */
+/* y[nrow] = alpha*A*x[ncol] + beta*y.  beta == 0 never reads y.  A launch
+ * captured in a CUDA graph stays valid until the plan is destroyed, whatever
+ * the plan is given in between (other configurations, a first SpMM). */
 int merbit_spmv(merbit_plan plan, double alpha, const void* d_x, double beta, void* d_y,
                 void* stream);
 

@@ -40,22 +40,32 @@ namespace {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-// Grows the plan's carry slots to `tiles` (both parity arrays start empty:
-// all ones).  The fill is ordered on s; callers synchronize s before a
-// launch on another stream can use the slots.
+// Gives the plan carry words for `tiles` tiles (both parity arrays start empty:
+// all ones).  A smaller block is kept, words and epoch, until the plan is
+// destroyed: a captured launch that holds its address stays valid.  The fill is
+// ordered on s; callers synchronize s before a launch on another stream can use
+// the words.
 int grow_carry(merbit_plan_s* p, int tiles, cudaStream_t s) {
-    if (tiles <= p->slots) return MERBIT_OK;
-    if (p->carry) {  // launches in flight may still use the old slots
-        MERBIT_CUDA(cudaDeviceSynchronize());
-        dev_free(p->carry, s);
-        p->carry = nullptr;
-        p->slots = 0;
-    }
-    const size_t words = 4 * (size_t)tiles;  // carries + boundary swaps, 2 parities
-    int st = dev_alloc(&p->carry, sizeof(unsigned long long) * words, s);
+    if (tiles <= p->carry.slots) return MERBIT_OK;
+    const bool first = p->carry.words == nullptr;  // takes the plan's own launch state
+    const size_t bytes = sizeof(unsigned long long) * 4 * (size_t)tiles;
+    SpmvCarry c;
+    int st = dev_alloc(&c.words, bytes + (first ? 0 : sizeof(LaunchState)), s);
     if (st != MERBIT_OK) return st;
-    MERBIT_CUDA(cudaMemsetAsync(p->carry, 0xFF, sizeof(unsigned long long) * words, s));
-    p->slots = tiles;
+    c.slots = tiles;
+    c.state = first ? p->state : reinterpret_cast<LaunchState*>(c.words + 4 * (size_t)tiles);
+    cudaError_t e = cudaMemsetAsync(c.words, 0xFF, bytes, s);
+    if (e == cudaSuccess && !first) {
+        LaunchState init = {};
+        init.epoch = 1u;
+        e = cudaMemcpyAsync(c.state, &init, sizeof(init), cudaMemcpyHostToDevice, s);
+    }
+    if (e != cudaSuccess) {
+        dev_free(c.words, s);
+        return cuda_fail(e, "carry slots");
+    }
+    if (!first) p->old_carries.push_back(p->carry);
+    p->carry = c;
     return MERBIT_OK;
 }
 
@@ -67,7 +77,6 @@ int plan_partition_start(merbit_plan_s* p, int tile_items, Partition** out, cuda
     Partition q;
     int st = build_partition_async(p->row_ptr, p->nrow, p->nnz, tile_items, &q,
                                    &p->scratch->max_rows, s);
-    if (st == MERBIT_OK) st = grow_carry(p, q.num_tiles, s);
     if (st != MERBIT_OK) {
         dev_free(q.coords, s);
         return st;
@@ -79,8 +88,6 @@ int plan_partition_start(merbit_plan_s* p, int tile_items, Partition** out, cuda
 
 }  // namespace
 
-// Ensures the plan holds a partition for `tile_items` and enough carry
-// slots; returns it in *out.  Synchronizes s when it builds one.
 int plan_partition(merbit_plan_s* p, int tile_items, const Partition** out, cudaStream_t s) {
     for (auto& q : p->parts)
         if (q.tile_items == tile_items) {
@@ -106,6 +113,18 @@ int plan_partition(merbit_plan_s* p, int tile_items, const Partition** out, cuda
 
 namespace {
 
+// The partition of an SpMV configuration, with carry words for its tiles.
+// (SpMM and batch launches bring words of their own, SpmmSlots, and take the
+// partition alone.)
+int spmv_partition(merbit_plan_s* p, int tile_items, const Partition** out, cudaStream_t s) {
+    int st = plan_partition(p, tile_items, out, s);
+    if (st != MERBIT_OK || (*out)->num_tiles <= p->carry.slots) return st;
+    st = grow_carry(p, (*out)->num_tiles, s);
+    if (st != MERBIT_OK) return st;
+    MERBIT_CUDA(cudaStreamSynchronize(s));
+    return MERBIT_OK;
+}
+
 // Whether configuration idx can run this plan (builds its partition).
 int plan_config_ok(merbit_plan_s* p, int idx, bool* ok, cudaStream_t s) {
     *ok = false;
@@ -116,7 +135,7 @@ int plan_config_ok(merbit_plan_s* p, int idx, bool* ok, cudaStream_t s) {
         return MERBIT_OK;
     }
     const Partition* part = nullptr;
-    int st = plan_partition(p, spmv_tile_items(c), &part, s);
+    int st = spmv_partition(p, spmv_tile_items(c), &part, s);
     if (st != MERBIT_OK) return st;
     *ok = part->max_rows <= spmv_config_row_cap(c);
     return MERBIT_OK;
@@ -182,11 +201,11 @@ int plan_partials(merbit_plan_s* p, int num_tiles, cudaStream_t s) {
     MERBIT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
     const long long need = std::max<long long>(num_tiles, 32LL * std::max(sms, 1));
     if (need <= p->npartials) return MERBIT_OK;
-    dev_free(p->partials, s);  // ordered after this plan's earlier launches
-    p->partials = nullptr;
-    p->npartials = 0;
-    int st = dev_alloc(&p->partials, sizeof(double) * (size_t)need, s);
+    double* words = nullptr;
+    int st = dev_alloc(&words, sizeof(double) * (size_t)need, s);
     if (st != MERBIT_OK) return st;
+    if (p->partials) p->owned.push_back(p->partials);  // captured launches may hold it
+    p->partials = words;
     p->npartials = need;
     return MERBIT_OK;
 }
@@ -199,7 +218,7 @@ int run_spmv(merbit_plan_s* p, int cfg, double alpha, const void* x, double beta
     const Partition* part = nullptr;
     int st = MERBIT_OK;
     if (c.kind != 3) {
-        st = plan_partition(p, spmv_tile_items(c), &part, s);
+        st = spmv_partition(p, spmv_tile_items(c), &part, s);
         if (st != MERBIT_OK) return st;
     }
     if (residual) {
@@ -213,10 +232,10 @@ int run_spmv(merbit_plan_s* p, int cfg, double alpha, const void* x, double beta
     a.x = x;
     a.y = y;
     a.coords = part ? part->coords : nullptr;
-    a.slots = p->carry;
-    a.xch = p->carry + 2 * (size_t)p->slots;
-    a.nslots = p->slots;
-    a.state = p->state;
+    a.slots = p->carry.words;
+    a.xch = p->carry.words + 2 * (size_t)p->carry.slots;
+    a.nslots = p->carry.slots;
+    a.state = part ? p->carry.state : p->state;  // row groups have no carries
     a.nrow = p->nrow;
     a.nnz = p->nnz;
     a.num_tiles = part ? part->num_tiles : 0;
@@ -412,6 +431,7 @@ int merbit_plan_create(merbit_plan* plan, int32_t nrow, int32_t ncol, int32_t nn
     Partition* part = nullptr;
     if (st == MERBIT_OK && first >= 0 && spmv_config(dtype, first).kind != 3)
         st = plan_partition_start(p, spmv_tile_items(spmv_config(dtype, first)), &part, s);
+    if (st == MERBIT_OK && part) st = grow_carry(p, part->num_tiles, s);
     PlanScratch h = {};
     if (st == MERBIT_OK) {
         e = cudaMemcpyAsync(&h, p->scratch, sizeof(h), cudaMemcpyDeviceToHost, s);
@@ -469,7 +489,8 @@ int merbit_plan_destroy(merbit_plan plan) {
         dev_free(kv.second.words, nullptr);
         dev_free(kv.second.state, nullptr);
     }
-    dev_free(plan->carry, nullptr);
+    dev_free(plan->carry.words, nullptr);
+    for (auto& c : plan->old_carries) dev_free(c.words, nullptr);
     dev_free(plan->state, nullptr);
     dev_free(plan->row_of, nullptr);
     dev_free(plan->partials, nullptr);
@@ -490,7 +511,9 @@ int merbit_plan_get_info(merbit_plan plan, merbit_plan_info* info) {
     info->items_per_thread = c.ipt;
     info->tile_items = spmv_tile_items(c);
     info->num_tiles = 0;
-    int64_t meta = sizeof(LaunchState) + (int64_t)plan->slots * 4 * (int64_t)sizeof(unsigned long long);
+    int64_t slots = plan->carry.slots;
+    for (auto& c : plan->old_carries) slots += c.slots;
+    int64_t meta = sizeof(LaunchState) + slots * 4 * (int64_t)sizeof(unsigned long long);
     for (auto& q : plan->parts) {
         if (q.tile_items == info->tile_items) info->num_tiles = q.num_tiles;
         meta += (int64_t)(q.num_tiles + 1) * (int64_t)sizeof(int2);
@@ -653,16 +676,29 @@ int merbit_plan_config_usable(merbit_plan plan, int32_t idx, int32_t* usable, vo
 int merbit_plan_check(merbit_plan plan, void* stream) {
     if (!plan) return fail(MERBIT_ERR_INVALID, "plan_check: plan is null");
     cudaStream_t s = (cudaStream_t)stream;
-    int err = 0;
-    MERBIT_CUDA(cudaMemcpyAsync(&err, &plan->state->error, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MERBIT_CUDA(cudaStreamSynchronize(s));
-    if (err != 0) {
+    auto take = [&](LaunchState* ls) -> int {  // reads and clears one state's error
+        int err = 0;
+        MERBIT_CUDA(cudaMemcpyAsync(&err, &ls->error, sizeof(int), cudaMemcpyDeviceToHost, s));
+        MERBIT_CUDA(cudaStreamSynchronize(s));
+        if (err == 0) return MERBIT_OK;
         const int zero = 0;
-        MERBIT_CUDA(cudaMemcpyAsync(&plan->state->error, &zero, sizeof(int), cudaMemcpyHostToDevice, s));
+        MERBIT_CUDA(cudaMemcpyAsync(&ls->error, &zero, sizeof(int), cudaMemcpyHostToDevice, s));
         MERBIT_CUDA(cudaStreamSynchronize(s));
         return fail(err, "a device-side carry wait ran out");
+    };
+    // the plan's launch state (also the first carry block's) and those of the
+    // blocks that followed
+    int st = take(plan->state);
+    if (plan->carry.state && plan->carry.state != plan->state) {
+        const int r = take(plan->carry.state);
+        if (st == MERBIT_OK) st = r;
     }
-    return MERBIT_OK;
+    for (auto& c : plan->old_carries) {
+        if (c.state == plan->state) continue;
+        const int r = take(c.state);
+        if (st == MERBIT_OK) st = r;
+    }
+    return st;
 }
 
 }  // extern "C"

@@ -418,6 +418,15 @@ struct SpmmSlots {
 };
 int alloc_spmm_slots(SpmmSlots* s, long long nslots, cudaStream_t st);
 
+// Carry and swap words of a plan's SpMV launches (2 parities x 2 arrays x
+// slots).  The epoch that selects the parity belongs to the words: launches on
+// another block do not turn this one's.
+struct SpmvCarry {
+    unsigned long long* words = nullptr;
+    LaunchState* state = nullptr;
+    int slots = 0;
+};
+
 // SpMV kernel configurations (spmv.cu).
 struct SpmvConfig {
     int kind;  // 0: CTA-tile kernel, 1: warp-tile kernel
@@ -666,10 +675,11 @@ struct merbit_plan_s {
     int cfg = 0;  // index into the SpMV config table
     int max_row_len = -1;  // longest row (-1: not measured)
     std::vector<merbit::Partition> parts;
-    // carry slots shared by every launch of this plan (2 * slots words,
-    // sized for the largest tile count in use)
-    unsigned long long* carry = nullptr;
-    int slots = 0;
+    // carry words of the merge-path SpMV launches, for the largest tile count
+    // in use, and the blocks that were too small for a later configuration:
+    // captured launches hold their addresses, so they live as long as the plan
+    merbit::SpmvCarry carry;
+    std::vector<merbit::SpmvCarry> old_carries;
     merbit::LaunchState* state = nullptr;
     merbit::PlanScratch* scratch = nullptr;  // same allocation as state
     // SpMM carry slots, keyed by (k << 20 | tile items)
@@ -686,5 +696,7 @@ struct merbit_plan_s {
 };
 
 namespace merbit {
+// The plan's partition for `tile_items` (coordinates alone; built, with one
+// synchronization of s, when the plan has none).
 int plan_partition(merbit_plan_s* p, int tile_items, const Partition** out, cudaStream_t s);
 }
