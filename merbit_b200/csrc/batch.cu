@@ -103,25 +103,39 @@ long long tile_cost(const merbit_plan_s* p, int items, int warps) {
     return tile_rounds(p, items, warps) * (items + kTileCost);
 }
 
-// No carry slots could be had for a kernel wider than the columns (under
-// capture, or out of memory): not a merbit_status.
-constexpr int kNoSlots = -1;
+// Operands of one SpMM launch: X, Y and, for a fused dval, dv_x and dv_out.
+struct SpmmOperands {
+    const void* x;
+    long long ldx;
+    void* y;
+    long long ldy;
+    const void* dv_x;
+    long long dv_ldx;
+    void* dv_out;
+};
 
-// One launch over columns [0, cols) of X / Y (pointers already offset), by the
-// kernel of kk >= cols columns.
-int spmm_block(merbit_plan_s* p, int kk, int cols, double alpha, const void* x, long long ldx, double beta,
-               void* y, long long ldy, cudaStream_t s, const void* dv_x = nullptr,
-               long long dv_ldx = 0, void* dv_out = nullptr) {
+// A launch over `cols` columns by the kernel of kk >= cols columns, at vector
+// width vw, in tiles of `items` merge items.
+struct SpmmShape {
+    int kk, cols, vw, items;
+};
+
+// Widest vector width the operands allow (with a fused dval, dv_x rows are
+// loaded with the same width).
+int spmm_width(const merbit_plan_s* p, int kk, int cols, int items, const SpmmOperands& o) {
     const int esz = (int)xy_size(p->dtype);
-    // vector width: the widest the operands allow (with a fused dval, dv_x
-    // rows are loaded with the same width)
-    auto width = [&](int items) {
-        int vw = pick_vw(kk, ldx, x, y, ldy, esz, items);
-        while (vw > 1 && cols % vw != 0) vw >>= 1;  // a lane's columns are all used or none
-        if (dv_out)
-            while (vw > 1 && (dv_ldx % vw != 0 || (uintptr_t)dv_x % ((size_t)vw * esz) != 0)) vw >>= 1;
-        return vw;
-    };
+    int vw = pick_vw(kk, o.ldx, o.x, o.y, o.ldy, esz, items);
+    while (vw > 1 && cols % vw != 0) vw >>= 1;  // a lane's columns are all used or none
+    if (o.dv_out)
+        while (vw > 1 && (o.dv_ldx % vw != 0 || (uintptr_t)o.dv_x % ((size_t)vw * esz) != 0)) vw >>= 1;
+    return vw;
+}
+
+// The shape of a launch over `cols` columns.
+SpmmShape spmm_shape(const merbit_plan_s* p, int cols, const SpmmOperands& o) {
+    int kk = 1;
+    while (kk < cols) kk <<= 1;
+    auto width = [&](int items) { return spmm_width(p, kk, cols, items, o); };
     // at vector width 4 (k >= 4) the larger tiles measured faster on the
     // power-law and banded matrices, and among them the one of an odd length
     // per lane group (480, 496, 504, 508 items at k = 4, 8, 16, 32: no bank
@@ -134,11 +148,10 @@ int spmm_block(merbit_plan_s* p, int kk, int cols, double alpha, const void* x, 
         items = 512;
         const int odd = spmm_odd_tile(kk);
         if (odd && width(odd) == 4) items = odd;
-    } else if (kk == 2 && !dv_out && width(352) == 2) {
+    } else if (kk == 2 && !o.dv_out && width(352) == 2) {
         items = 352;
     }
     int vw = width(items);
-    if (!spmm_config_exists(kk, vw, items)) return MERBIT_ERR_UNSUPPORTED;
     // Vector width 2 in tiles of an odd length per lane group: where the operands
     // allow no more (FP32 k = 6: 95 us against 109 in 256-item tiles; R-MAT-300k),
     // and in FP64, whose 16-byte loads then take a lane's whole slice and half
@@ -146,7 +159,7 @@ int spmm_block(merbit_plan_s* p, int kk, int cols, double alpha, const void* x, 
     // against 190; on an 80 x 70 x 60 27-point stencil k = 8 98 against 120, k = 32
     // 209 against 250; on Zipf-300k k = 32 227 against 301.  Not at 9 to 16 columns:
     // k = 16 on Zipf-300k takes 152 us against 129.
-    if (!dv_out && kk >= 4 && (vw == 2 || (vw == 4 && p->dtype == MERBIT_F64 && kk != 16))) {
+    if (!o.dv_out && kk >= 4 && (vw == 2 || (vw == 4 && p->dtype == MERBIT_F64 && kk != 16))) {
         items = spmm_odd_tile2(kk);
         vw = 2;
     }
@@ -163,36 +176,62 @@ int spmm_block(merbit_plan_s* p, int kk, int cols, double alpha, const void* x, 
         if ((kk >= 16 || one_round) && tile_cost(p, small, warps) < tile_cost(p, items, warps))
             items = small;
     }
-    const Partition* part = nullptr;
-    int st = plan_partition(p, items, &part, s);
-    if (st != MERBIT_OK) return cols < kk ? kNoSlots : st;
-    const long long key = ((long long)kk << 20) | items;
-    auto it = p->spmm_slots.find(key);
-    if (it == p->spmm_slots.end()) {
-        SpmmSlots sl;
-        st = alloc_spmm_slots(&sl, (long long)part->num_tiles * kk, s);
-        if (st != MERBIT_OK) return cols < kk ? kNoSlots : st;
-        it = p->spmm_slots.emplace(key, sl).first;
+    return {kk, cols, vw, items};
+}
+
+long long slot_key(const SpmmShape& h) { return ((long long)h.kk << 20) | h.items; }
+
+// Makes the partition and the carry slots of a shape when the plan has none.
+// *room tells a failure apart that another shape may avoid: s is being captured
+// (nothing is queued then), or there is no memory.
+int spmm_reserve(merbit_plan_s* p, const SpmmShape& h, cudaStream_t s, bool* room) {
+    *room = true;
+    if (p->spmm_slots.count(slot_key(h))) return MERBIT_OK;  // made after their partition
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    MERBIT_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+        *room = false;
+        return fail(MERBIT_ERR_INVALID,
+                    "spmm: the stream is being captured and the plan has no carry slots for this "
+                    "call: make the same call (k, leading dimensions, alignment) before capture");
     }
+    const Partition* part = nullptr;
+    int st = plan_partition(p, h.items, &part, s);
+    if (st == MERBIT_OK) {
+        SpmmSlots sl;
+        st = alloc_spmm_slots(&sl, (long long)part->num_tiles * h.kk, s);
+        if (st == MERBIT_OK) p->spmm_slots.emplace(slot_key(h), sl);
+    }
+    if (st != MERBIT_OK) *room = !out_of_memory();
+    return st;
+}
+
+// The launch, its slots reserved.
+int spmm_run(merbit_plan_s* p, const SpmmShape& h, const SpmmOperands& o, double alpha, double beta,
+             cudaStream_t s) {
+    const Partition* part = nullptr;
+    int st = plan_partition(p, h.items, &part, s);  // there
+    if (st != MERBIT_OK) return st;
+    const SpmmSlots& sl = p->spmm_slots.find(slot_key(h))->second;
     SpmmLaunch a = {};
-    a.single = make_desc(p, part, x, ldx, y, ldy, 0);
+    a.single = make_desc(p, part, o.x, o.ldx, o.y, o.ldy, 0);
     a.descs = nullptr;
     a.ndesc = 0;
-    a.nslots = (int)it->second.nslots;
-    a.slots = it->second.words;
-    a.xch = it->second.words + 2 * (size_t)it->second.nslots;
-    a.state = it->second.state;
+    a.nslots = (int)sl.nslots;
+    a.slots = sl.words;
+    a.xch = sl.words + 2 * (size_t)sl.nslots;
+    a.state = sl.state;
     a.total_tiles = part->num_tiles;
-    a.cols = cols;
+    a.cols = h.cols;
     a.alpha = alpha;
     a.beta = beta;
-    if (dv_out) {
-        a.dv_x = dv_x;
-        a.dv_ldx = dv_ldx;
+    if (o.dv_out) {
+        a.dv_x = o.dv_x;
+        a.dv_ldx = o.dv_ldx;
         a.dv_perm = p->perm;
-        a.dv_out = dv_out;
+        a.dv_out = o.dv_out;
     }
-    return spmm_launch(p->dtype, kk, vw, items, a, s);
+    return spmm_launch(p->dtype, h.kk, h.vw, h.items, a, s);
 }
 
 }  // namespace
@@ -414,18 +453,18 @@ int merbit_spmm(merbit_plan plan, int32_t k, double alpha, const void* d_x, int6
     // 175, 153 and 252; no k from 2 to 40 is faster split.
     int j = 0;
     while (j < k) {
-        int cols = k - j < 32 ? k - j : 32;
-        int kk = 1;
-        while (kk < cols) kk <<= 1;
-        const char* xb = static_cast<const char*>(d_x) + (size_t)j * esz;
-        char* yb = static_cast<char*>(d_y) + (size_t)j * esz;
-        int st = spmm_block(plan, kk, cols, alpha, xb, ldx, beta, yb, ldy, s);
-        if (st == kNoSlots) {  // as many columns as a narrower kernel's own
-            cols = kk = kk >> 1;
-            st = spmm_block(plan, kk, cols, alpha, xb, ldx, beta, yb, ldy, s);
+        const SpmmOperands o = {static_cast<const char*>(d_x) + (size_t)j * esz, ldx,
+                                static_cast<char*>(d_y) + (size_t)j * esz, ldy, nullptr, 0, nullptr};
+        SpmmShape h = spmm_shape(plan, std::min(k - j, 32), o);
+        bool room = true;
+        int st = spmm_reserve(plan, h, s, &room);
+        if (!room && h.cols < h.kk) {  // as many columns as a narrower kernel's own
+            h = spmm_shape(plan, h.kk >> 1, o);
+            st = spmm_reserve(plan, h, s, &room);
         }
+        if (st == MERBIT_OK) st = spmm_run(plan, h, o, alpha, beta, s);
         if (st != MERBIT_OK) return st;
-        j += cols;
+        j += h.cols;
     }
     return MERBIT_OK;
 }
@@ -443,11 +482,12 @@ int merbit_spmm_dval(merbit_plan tplan, int32_t k, const void* d_g, int64_t ldg,
     if (tplan->nrow == 0) return MERBIT_OK;
     if (!d_dx || !d_dval || (tplan->ncol > 0 && !d_g) || !d_x)
         return fail(MERBIT_ERR_INVALID, "spmm_dval: null pointer");
-    const int st = spmm_block(tplan, k, k, 1.0, d_g, ldg, 0.0, d_dx, lddx, (cudaStream_t)stream, d_x,
-                              ldx, d_dval);
-    if (st == MERBIT_ERR_UNSUPPORTED)
-        return fail(MERBIT_ERR_UNSUPPORTED, "spmm_dval: no configuration for these operands");
-    return st;
+    cudaStream_t s = (cudaStream_t)stream;
+    const SpmmOperands o = {d_g, ldg, d_dx, lddx, d_x, ldx, d_dval};
+    const SpmmShape h = spmm_shape(tplan, k, o);
+    bool room = true;
+    const int st = spmm_reserve(tplan, h, s, &room);
+    return st == MERBIT_OK ? spmm_run(tplan, h, o, 1.0, 0.0, s) : st;
 }
 
 int merbit_batch_create(merbit_batch* batch, int32_t count, const merbit_plan* plans, int32_t k,

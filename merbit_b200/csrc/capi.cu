@@ -17,17 +17,20 @@ namespace merbit {
 namespace {
 thread_local std::string g_detail;
 thread_local int g_last_cuda = 0;
+thread_local bool g_no_memory = false;
 }  // namespace
 
 void set_error_detail(const std::string& s) { g_detail = s; }
 
 int fail(int status, const std::string& detail) {
     g_detail = detail;
+    g_no_memory = false;
     return status;
 }
 
 int cuda_fail(cudaError_t e, const char* where) {
     g_last_cuda = (int)e;
+    g_no_memory = e == cudaErrorMemoryAllocation;
     g_detail = std::string(where) + ": " + cudaGetErrorString(e);
     // un-latch a non-sticky error so that a later launch check of this
     // thread does not report it again (a sticky error stays)
@@ -35,6 +38,7 @@ int cuda_fail(cudaError_t e, const char* where) {
     return MERBIT_ERR_CUDA;
 }
 
+bool out_of_memory() { return g_no_memory; }
 
 namespace {
 
@@ -73,7 +77,6 @@ int grow_carry(merbit_plan_s* p, int tiles, cudaStream_t s) {
 // rows-per-tile lands in p->scratch->max_rows for the caller's next
 // readback.  On failure nothing is added to the plan.
 int plan_partition_start(merbit_plan_s* p, int tile_items, Partition** out, cudaStream_t s) {
-    MERBIT_CUDA(cudaMemsetAsync(&p->scratch->max_rows, 0, sizeof(int), s));
     Partition q;
     int st = build_partition_async(p->row_ptr, p->nrow, p->nnz, tile_items, &q,
                                    &p->scratch->max_rows, s);

@@ -343,6 +343,7 @@ __device__ __forceinline__ void st4_shared(float* p, const float (&v)[4]) {
 void set_error_detail(const std::string& s);
 int fail(int status, const std::string& detail);
 int cuda_fail(cudaError_t e, const char* where);
+bool out_of_memory();  // whether this thread's last failure was a refused allocation
 
 #define MERBIT_CUDA(call)                                          \
     do {                                                           \
@@ -380,9 +381,8 @@ struct Partition {
 constexpr int warp_rp_cap(int ipt) { return (32 * ipt) / 3 + 16; }
 
 // Allocates out->coords and queues the merge-path search of every tile
-// boundary on s, without synchronizing; the largest rows-per-tile is
-// atomically maxed into *d_max_rows (zeroed by the caller), and
-// out->max_rows stays -1 until the caller reads it back.
+// boundary on s, without synchronizing; the largest rows-per-tile lands in
+// *d_max_rows, and out->max_rows stays -1 until the caller reads it back.
 int build_partition_async(const int32_t* row_ptr, int nrow, int nnz, int tile_items,
                           Partition* out, int* d_max_rows, cudaStream_t s);
 

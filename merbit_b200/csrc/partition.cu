@@ -153,8 +153,10 @@ int build_partition_async(const int32_t* row_ptr, int nrow, int nnz, int tile_it
     out->tile_items = tile_items;
     out->num_tiles = (int)T;
     out->max_rows = -1;
+    // before anything is queued: it is refused while s is being captured
     int st = dev_alloc(&out->coords, sizeof(int2) * (size_t)(T + 1), s);
     if (st != MERBIT_OK) return st;
+    MERBIT_CUDA(cudaMemsetAsync(d_max_rows, 0, sizeof(int), s));
     const long long count = T + 1;
     const int bs = 256;
     const unsigned grid = (unsigned)((count + bs - 1) / bs);
