@@ -53,7 +53,7 @@ def _hostcxx() -> str:
 
 
 def _headers() -> list[str]:
-    return glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    return glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
 
 
 def _digest(files: list[str], extra: list[str]) -> str:

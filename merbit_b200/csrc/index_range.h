@@ -1,0 +1,23 @@
+// Index arithmetic of the kernels at the top of the accepted range (nrow + nnz
+// up to INT_MAX - 64), in plain C++ so that it can also be run on the host.
+#pragma once
+
+#ifdef __CUDACC__
+#define MERBIT_HD __host__ __device__ __forceinline__
+#else
+#define MERBIT_HD inline
+#endif
+
+namespace merbit {
+
+// The SpMM walk counts nonzeros as in the whole matrix, and all lanes of a warp
+// take as many steps as the longest of its segments.  A lane group that is done
+// stays at the end of its own segment: what it looks ahead from there (two
+// chunks, 16 nonzeros at most) is within the 64 that the plan keeps free.
+MERBIT_HD int walk_next(int c, int by, int end) { return c + by < end ? c + by : end; }
+// nonzero c + t of a chunk; past the segment's end one of the tile again
+MERBIT_HD int walk_entry(int c, int t, int last) { return c + t < last ? c + t : last; }
+// whether no row or segment ends at or before nonzero c + n
+MERBIT_HD bool walk_clear(int lim, int c, int n) { return lim > c + n; }
+
+}  // namespace merbit

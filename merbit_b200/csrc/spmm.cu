@@ -43,6 +43,7 @@
 // permutation (staged by TMA with the tile's col and vals).
 #include <type_traits>
 
+#include "index_range.h"
 #include "merbit_internal.cuh"
 
 namespace merbit {
@@ -709,7 +710,7 @@ struct SpmmTile {
         auto load_chunk = [&](int c, XRow<X, VW> (&xr)[CH], V (&vv)[CH]) {
 #pragma unroll
             for (int t = 0; t < CH; ++t) {
-                const int e = min(c + t, e_last);
+                const int e = walk_entry(c, t, e_last);
                 const unsigned colv = (unsigned)col_t[e];
                 vv[t] = val_t[e];
                 xr[t].load(reinterpret_cast<const X*>(xl + (unsigned long long)colv * xstep));
@@ -719,7 +720,7 @@ struct SpmmTile {
         // or before c is finished, so c belongs to row ly.  Called by all
         // lanes of the warp.
         auto consume = [&](int c, const XRow<X, VW> (&xr)[CH], const V (&vv)[CH]) {
-            if (__all_sync(0xFFFFFFFFu, lim > c + CH)) {  // no row or segment ends here
+            if (__all_sync(0xFFFFFFFFu, walk_clear(lim, c, CH))) {  // no row or segment ends here
                 if constexpr (CH == 2) {
                     // F32/BF16: one compensated addition of the fused pair
                     acc.add_two(to_p(vv[0]), xr[0], to_p(vv[1]), xr[1]);
@@ -809,7 +810,7 @@ struct SpmmTile {
                 consume(c, xa, va);
                 load_chunk(c + 2 * CH, xa, va);
                 consume(c + CH, xb, vb);
-                c += 2 * CH;
+                c = walk_next(c, 2 * CH, lx_end);
             }
         }
 
