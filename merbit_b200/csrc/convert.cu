@@ -28,28 +28,28 @@ int grid_of(long long n) {
 
 __global__ void pack_keys(const int* __restrict__ major, const int* __restrict__ minor, int n,
                           unsigned long long* __restrict__ key, int* __restrict__ idx) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    each_index((unsigned)n, [&](int i) {
         key[i] = ((unsigned long long)(unsigned)major[i] << 32) | (unsigned)minor[i];
         idx[i] = i;
-    }
+    });
 }
 
 __global__ void unpack_keys(const unsigned long long* __restrict__ key, int n,
                             int* __restrict__ major, int* __restrict__ minor) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    each_index((unsigned)n, [&](int i) {
         major[i] = (int)(key[i] >> 32);
         minor[i] = (int)(key[i] & 0xFFFFFFFFull);
-    }
+    });
 }
 
 // Largest index of each array, as unsigned values.
 __global__ void max_indices(const int* __restrict__ major, const int* __restrict__ minor, int n,
                             unsigned* __restrict__ out) {
     unsigned a = 0u, b = 0u;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    each_index((unsigned)n, [&](int i) {
         a = max(a, (unsigned)major[i]);
         b = max(b, (unsigned)minor[i]);
-    }
+    });
     a = __reduce_max_sync(0xFFFFFFFFu, a);
     b = __reduce_max_sync(0xFFFFFFFFu, b);
     if ((threadIdx.x & 31) == 0) {
@@ -61,9 +61,10 @@ __global__ void max_indices(const int* __restrict__ major, const int* __restrict
 // One word per triplet: major, minor (b_minor bits) and position (b_pos bits).
 __global__ void pack_words(const int* __restrict__ major, const int* __restrict__ minor, int n,
                            int b_minor, int b_pos, unsigned long long* __restrict__ word) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    each_index((unsigned)n, [&](int i) {
         word[i] = ((((unsigned long long)(unsigned)major[i] << b_minor) | (unsigned)minor[i]) << b_pos) |
                   (unsigned)i;
+    });
 }
 
 template <typename V>
@@ -71,12 +72,12 @@ __global__ void unpack_words(const unsigned long long* __restrict__ word, int n,
                              int b_pos, int* __restrict__ major, int* __restrict__ minor,
                              const V* __restrict__ src, V* __restrict__ dst) {
     const unsigned long long pos = (1ull << b_pos) - 1, min_mask = (1ull << b_minor) - 1;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    each_index((unsigned)n, [&](int i) {
         const unsigned long long w = word[i];
         major[i] = (int)(w >> (b_minor + b_pos));
         minor[i] = (int)((w >> b_pos) & min_mask);
         if (src) dst[i] = src[w & pos];
-    }
+    });
 }
 
 int bits_of(unsigned long long v) {
@@ -88,35 +89,34 @@ int bits_of(unsigned long long v) {
 template <typename V>
 __global__ void permute_vals(const V* __restrict__ src, const int* __restrict__ perm, int n,
                              V* __restrict__ dst) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        dst[i] = src[perm[i]];
+    each_index((unsigned)n, [&](int i) { dst[i] = src[perm[i]]; });
 }
 
 // offsets[r] = first position with sorted[pos] >= r, r in [0, nrow].
 __global__ void offsets_kernel(const int* __restrict__ sorted, int n, int nrow,
                                int* __restrict__ offsets) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= n; j += gridDim.x * blockDim.x) {
-        const int prev = j == 0 ? -1 : min(sorted[j - 1], nrow);
+    each_index((unsigned)n + 1u, [&](int j) {
+        const int prev = j == 0 ? -1 : max(min(sorted[j - 1], nrow), -1);
         const int cur = j == n ? nrow : min(sorted[j], nrow);
-        for (int r = prev + 1; r <= cur; ++r) offsets[r] = j;
-    }
+        for (long long r = (long long)prev + 1; r <= cur; ++r) offsets[r] = j;
+    });
 }
 
 // cnt[nrow] counts indices outside [0, nrow).
 __global__ void count_kernel(const int* __restrict__ idx, int n, int nrow, int* __restrict__ cnt) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    each_index((unsigned)n, [&](int i) {
         const int r = idx[i];
         atomicAdd(cnt + ((unsigned)r < (unsigned)nrow ? r : nrow), 1);
-    }
+    });
 }
 
 template <typename V>
 __global__ void inv_count_kernel(const int* __restrict__ idx, const int* __restrict__ cnt, int n,
                                  int nrow, V* __restrict__ vals) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    each_index((unsigned)n, [&](int i) {
         const int r = idx[i];
         vals[i] = (V)((unsigned)r < (unsigned)nrow ? 1.0 / (double)cnt[r] : 0.0);
-    }
+    });
 }
 
 }  // namespace

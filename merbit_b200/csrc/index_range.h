@@ -20,4 +20,12 @@ MERBIT_HD int walk_entry(int c, int t, int last) { return c + t < last ? c + t :
 // whether no row or segment ends at or before nonzero c + n
 MERBIT_HD bool walk_clear(int lim, int c, int n) { return lim > c + n; }
 
+
+// f(i) for i = first, first + stride, ... below n: unsigned, as the last step
+// passes n by up to a grid's threads (1.2 million) and n may be INT_MAX (+ 1)
+template <class F>
+MERBIT_HD void strided(unsigned first, unsigned stride, unsigned n, F&& f) {
+    for (unsigned i = first; i < n; i += stride) f((int)i);
+}
+
 }  // namespace merbit

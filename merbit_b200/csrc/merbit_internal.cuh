@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/merbit.h"
+#include "index_range.h"
 
 namespace merbit {
 
@@ -237,6 +238,12 @@ __device__ __forceinline__ double look_back(const unsigned long long* slots, int
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
     return sum;
+}
+
+// f(i) for i < n, over the threads of a grid.
+template <class F>
+__device__ __forceinline__ void each_index(unsigned n, F&& f) {
+    strided(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, n, f);
 }
 
 // ---------------------------------------------------------------------------

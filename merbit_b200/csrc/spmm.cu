@@ -43,7 +43,6 @@
 // permutation (staged by TMA with the tile's col and vals).
 #include <type_traits>
 
-#include "index_range.h"
 #include "merbit_internal.cuh"
 
 namespace merbit {

@@ -16,14 +16,13 @@ namespace merbit {
 namespace {
 
 __global__ void iota_kernel(int* __restrict__ out, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] = i;
+    each_index((unsigned)n, [&](int i) { out[i] = i; });
 }
 
 // row_of[e] = r with row_ptr[r] <= e < row_ptr[r+1] (upper bound - 1).
 __global__ void row_of_kernel(const int32_t* __restrict__ row_ptr, int nrow, int nnz,
                               int* __restrict__ row_of) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
+    each_index((unsigned)nnz, [&](int e) {
         int lo = 0, hi = nrow;  // find largest r with row_ptr[r] <= e
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
@@ -34,31 +33,29 @@ __global__ void row_of_kernel(const int32_t* __restrict__ row_ptr, int nrow, int
         }
         // skip empty rows sharing the same start
         row_of[e] = lo;
-    }
+    });
 }
 
 // col_ptr from the sorted column keys: col_ptr[c] = first j with key[j] >= c.
 __global__ void col_ptr_kernel(const int* __restrict__ key, int nnz, int ncol,
                                int* __restrict__ col_ptr) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= nnz; j += gridDim.x * blockDim.x) {
+    each_index((unsigned)nnz + 1u, [&](int j) {
         const int prev = j == 0 ? -1 : key[j - 1];
         const int cur = j == nnz ? ncol : key[j];
-        for (int c = prev + 1; c <= cur; ++c) col_ptr[c] = j;
-    }
+        for (long long c = (long long)prev + 1; c <= cur; ++c) col_ptr[c] = j;
+    });
 }
 
 template <typename V>
 __global__ void gather_kernel(const V* __restrict__ src, const int* __restrict__ perm, int n,
                               V* __restrict__ dst) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-        dst[j] = src[perm[j]];
+    each_index((unsigned)n, [&](int j) { dst[j] = src[perm[j]]; });
 }
 
 template <typename T>
 __global__ void gather_map_kernel(const int* __restrict__ src, const int* __restrict__ perm,
                                   int n, int* __restrict__ dst) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-        dst[j] = src[perm[j]];
+    each_index((unsigned)n, [&](int j) { dst[j] = src[perm[j]]; });
 }
 
 int grid_for(long long n) {

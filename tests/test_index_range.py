@@ -75,6 +75,34 @@ int main() {
 }
 """
 
+STRIDED = r"""
+#include <climits>
+#include <cstdio>
+#include <initializer_list>
+#include "index_range.h"
+using namespace merbit;
+
+int main() {
+    const unsigned stride = 148u * 32u * 256u;  // the largest grid of the conversions
+    for (unsigned n : {0u, 1u, stride, (unsigned)INT_MAX - stride, (unsigned)INT_MAX - 1u,
+                       (unsigned)INT_MAX, (unsigned)INT_MAX + 1u})
+        for (unsigned first : {0u, 1u, 255u, stride - 1u}) {
+            unsigned long long calls = 0;
+            bool ok = true;
+            strided(first, stride, n, [&](int i) {
+                ok = ok && i >= 0 && (unsigned)i < n && (unsigned)i == first + calls * stride;
+                ++calls;
+            });
+            const unsigned long long want = n > first ? (n - first + (unsigned long long)stride - 1) / stride : 0;
+            if (!ok || calls != want) {
+                std::printf("n %u first %u: %llu calls, %llu expected\n", n, first, calls, want);
+                return 1;
+            }
+        }
+    return 0;
+}
+"""
+
 
 def _run(tmp_path, source):
     cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else shutil.which("g++")
@@ -91,3 +119,7 @@ def _run(tmp_path, source):
 
 def test_spmm_walk_at_the_largest_nonzero_count(tmp_path):
     _run(tmp_path, WALK)
+
+
+def test_grid_stride_loops_at_the_largest_count(tmp_path):
+    _run(tmp_path, STRIDED)
