@@ -28,4 +28,8 @@ MERBIT_HD void strided(unsigned first, unsigned stride, unsigned n, F&& f) {
     for (unsigned i = first; i < n; i += stride) f((int)i);
 }
 
+// Row groups: whether entry i + ahead of a row or staged run lies before its
+// end (unsigned: a lane looks up to 480 entries past the last one)
+MERBIT_HD bool before_end(unsigned i, unsigned ahead, int end) { return i + ahead < (unsigned)end; }
+
 }  // namespace merbit

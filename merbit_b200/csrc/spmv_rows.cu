@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(WARPS * 32) spmv_rows_kernel(const SpmvLaunch 
     constexpr int CAP = 32 * UNR;
     __shared__ P s_prod[STG ? WARPS : 1][STG ? CAP : 1];
     P* __restrict__ sp = s_prod[STG ? (threadIdx.x >> 5) : 0];
-    for (int r0 = gw * RPW; r0 < a.nrow; r0 += nw * RPW) {
-        const int r = r0 + grp;
+    for (unsigned r0 = gw * RPW; before_end(r0, 0u, a.nrow); r0 += nw * RPW) {
+        const int r = (int)r0 + grp;
         Acc acc;
         acc.zero();
         bool staged = false;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(WARPS * 32) spmv_rows_kernel(const SpmvLaunch 
                 s = __ldg(rp + r);
                 e = __ldg(rp + r + 1);
             }
-            const int nb_rows = min(RPW, a.nrow - r0);  // >= 1: r0 < nrow
+            const int nb_rows = min(RPW, a.nrow - (int)r0);  // >= 1: r0 < nrow
             const int bs = __shfl_sync(0xFFFFFFFFu, s, 0);
             const int be = __shfl_sync(0xFFFFFFFFu, e, (nb_rows - 1) * LPR);
             if (be - bs <= CAP) {  // warp-uniform
@@ -118,9 +118,10 @@ __global__ void __launch_bounds__(WARPS * 32) spmv_rows_kernel(const SpmvLaunch 
                 V v[UNR];
 #pragma unroll
                 for (int u = 0; u < UNR; ++u) {
-                    const int k = bs + lane + 32 * u;
-                    c[u] = k < be ? __ldcs(col + k) : -1;
-                    v[u] = k < be ? __ldcs(vals + k) : V(0);
+                    const unsigned k = (unsigned)(bs + lane);  // + 32 u
+                    const bool in = before_end(k, 32u * u, be);
+                    c[u] = in ? __ldcs(col + k + 32u * u) : -1;
+                    v[u] = in ? __ldcs(vals + k + 32u * u) : V(0);
                 }
                 X xg[UNR];
 #pragma unroll
@@ -147,14 +148,14 @@ __global__ void __launch_bounds__(WARPS * 32) spmv_rows_kernel(const SpmvLaunch 
             const int s = __ldg(rp + r), e = __ldg(rp + r + 1);
             // steps of UNR * LPR nonzeros, predicated at the row end, so all
             // of a step's loads are in flight together
-            for (int i = s + jl; i < e; i += UNR * LPR) {
+            for (unsigned i = (unsigned)(s + jl); before_end(i, 0u, e); i += UNR * LPR) {
                 int c[UNR];
                 V v[UNR];
 #pragma unroll
                 for (int u = 0; u < UNR; ++u) {
-                    const int k = i + u * LPR;
-                    c[u] = k < e ? __ldcs(col + k) : -1;
-                    v[u] = k < e ? __ldcs(vals + k) : V(0);
+                    const bool in = before_end(i, u * LPR, e);
+                    c[u] = in ? __ldcs(col + i + u * LPR) : -1;
+                    v[u] = in ? __ldcs(vals + i + u * LPR) : V(0);
                 }
                 X xg[UNR];
 #pragma unroll

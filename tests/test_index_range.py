@@ -103,6 +103,51 @@ int main() {
 }
 """
 
+ROWS = r"""
+#include <climits>
+#include <cstdio>
+#include <initializer_list>
+#include "index_range.h"
+using namespace merbit;
+
+// Every lane of a row group takes the row's entries once and none beyond it.
+static bool row(int s, int e, int lpr, int unr) {
+    long long taken = 0;
+    for (int jl = 0; jl < lpr; ++jl)
+        for (unsigned i = (unsigned)(s + jl); before_end(i, 0u, e); i += unr * lpr)
+            for (int u = 0; u < unr; ++u)
+                if (before_end(i, u * lpr, e)) {
+                    const unsigned k = i + u * lpr;
+                    if (k < (unsigned)s || k >= (unsigned)e) return false;
+                    ++taken;
+                }
+    return taken == e - s;
+}
+// ... and a warp those of a staged run of at most 32 * unr.
+static bool run(int bs, int be, int unr) {
+    long long taken = 0;
+    for (int lane = 0; lane < 32; ++lane)
+        for (int u = 0; u < unr; ++u)
+            if (before_end((unsigned)(bs + lane), 32u * u, be)) {
+                const unsigned k = (unsigned)(bs + lane) + 32u * u;
+                if (k < (unsigned)bs || k >= (unsigned)be) return false;
+                ++taken;
+            }
+    return taken == be - bs;
+}
+
+int main() {
+    for (int e : {INT_MAX - 65, INT_MAX - 66, INT_MAX - 300, 1000})
+        for (int len : {0, 1, 31, 32, 33, 500, 512})
+            for (int unr : {4, 8, 16}) {
+                for (int lpr : {1, 2, 4, 8, 16, 32})
+                    if (!row(e - len, e, lpr, unr)) return std::printf("row %d of %d, %d lanes\n", e, len, lpr), 1;
+                if (len <= 32 * unr && !run(e - len, e, unr)) return std::printf("run %d of %d\n", e, len), 1;
+            }
+    return 0;
+}
+"""
+
 
 def _run(tmp_path, source):
     cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else shutil.which("g++")
@@ -123,3 +168,7 @@ def test_spmm_walk_at_the_largest_nonzero_count(tmp_path):
 
 def test_grid_stride_loops_at_the_largest_count(tmp_path):
     _run(tmp_path, STRIDED)
+
+
+def test_row_groups_at_the_largest_nonzero_count(tmp_path):
+    _run(tmp_path, ROWS)
