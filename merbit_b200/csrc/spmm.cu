@@ -650,20 +650,20 @@ struct SpmmTile {
         }
         next_row(lx);
 
-        // fused dval: this lane's VW values of dv_x's current row.  (Loading
-        // the row after it ahead, or one shuffle tree for two nonzeros, was no
-        // faster: Zipf-1M FP32 at k = 16 took 542 and 539 us against 537.  The
-        // scattered dval writes bind this form: their 97 MB and G's 64 MB
-        // do not fit L2 together.)
+        // fused dval: this lane's VW values of dv_x's current row, loaded when
+        // the segment has a nonzero of it.  (Loading the row after it ahead, or
+        // one shuffle tree for two nonzeros, was no faster: Zipf-1M FP32 at k = 16
+        // took 542 and 539 us against 537.  The scattered dval writes bind this
+        // form: their 97 MB and G's 64 MB do not fit L2 together.)
         const int* perm_t = reinterpret_cast<const int*>(ws + perm_offset) - (x0 & ~3);
         XRow<X, VW> xrow;
-        auto dv_row = [&]() {  // ly is the current row
-            if (y0 + ly < nrow)
+        auto dv_row = [&](int e) {  // ly is the current row, e the next nonzero
+            if (e < lx_end)
                 xrow.load(static_cast<const X*>(a.dv_x) + (size_t)(y0 + ly) * a.dv_ldx + j0);
         };
         if (DV) {
             xrow.zero();
-            dv_row();
+            dv_row(lx);
         }
         const unsigned gmask = LPG == 32 ? 0xFFFFFFFFu : (((1u << LPG) - 1u) << (g * LPG));
         // dval of nonzero e: in the x type, VW fused multiply-adds per lane, then
@@ -696,7 +696,7 @@ struct SpmmTile {
             acc.zero();
             ++ly;
             next_row(e);
-            if (DV) dv_row();
+            if (DV) dv_row(e);
         };
 
         // ---- walk: chunks of CH nonzeros, the next chunk's x rows in flight
@@ -802,12 +802,16 @@ struct SpmmTile {
         } else {
             // as many steps for every lane: the longest segment's
             const int steps = __reduce_max_sync(0xFFFFFFFFu, (lx_end - lx + 2 * CH - 1) / (2 * CH));
+            // The last step loads no chunk beyond it where segments are short, a few
+            // steps each (k = 1: 5% less time); on longer ones the branch costs more
+            // than the load, and plain FP64 products would pass 96 registers.
+            constexpr bool kLastLoad = K >= 16 || (DT == MERBIT_F64 && !DV);
             int c = lx;
             if (steps > 0) load_chunk(c, xa, va);
-            for (int i = 0; i < steps; ++i) {
+            for (int i = 1; i <= steps; ++i) {
                 load_chunk(c + CH, xb, vb);
                 consume(c, xa, va);
-                load_chunk(c + 2 * CH, xa, va);
+                if (kLastLoad || i < steps) load_chunk(c + 2 * CH, xa, va);  // warp-uniform
                 consume(c + CH, xb, vb);
                 c = walk_next(c, 2 * CH, lx_end);
             }
