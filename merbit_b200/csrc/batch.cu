@@ -78,29 +78,26 @@ SpmmDesc make_desc(merbit_plan_s* p, const Partition* part, const void* x, long 
     return d;
 }
 
-// Warps of the SpMM kernel that the device holds: 5 CTAs of 4 per SM.
-int spmm_warps() {
+int device_sms() {
     static int sms[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return 148 * 20;
+    if (dev < 0 || dev >= 64) return 148;
     int n = __atomic_load_n(&sms[dev], __ATOMIC_RELAXED);
     if (n == 0) {
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
         __atomic_store_n(&sms[dev], n, __ATOMIC_RELAXED);
     }
-    return 20 * n;
+    return n;
 }
 
 // What a launch with tiles of `items` merge items takes, in items: the rounds
 // of its busiest warp, each tile costing about kTileCost items beyond its own.
 constexpr int kTileCost = 100;
-long long tile_rounds(const merbit_plan_s* p, int items, int warps) {
+long long tile_rounds(const merbit_plan_s* p, int kk, int vw, int items, bool dv) {
     const long long tiles = ((long long)p->nrow + p->nnz + items - 1) / items;
+    const int warps = spmm_resident_warps(p->dtype, kk, vw, items, dv, device_sms());
     return (tiles + warps - 1) / warps;
-}
-long long tile_cost(const merbit_plan_s* p, int items, int warps) {
-    return tile_rounds(p, items, warps) * (items + kTileCost);
 }
 
 // Operands of one SpMM launch: X, Y and, for a fused dval, dv_x and dv_out.
@@ -168,12 +165,14 @@ SpmmShape spmm_shape(const merbit_plan_s* p, int cols, const SpmmOperands& o) {
     // one round at most (beyond, its overhead was seen to cost up to 15%), for more
     // columns whenever its rounds cost less.  R-MAT of degree 30, us, larger / smaller
     // tile: 2,000 rows FP32 k = 4, 16, 32 13 / 12, 22 / 16, 32 / 20; 20,000 rows FP64
-    // k = 8 28 / 21; 60,000 rows FP32 k = 32 58 / 51.
+    // k = 8 28 / 21; 60,000 rows FP32 k = 32 58 / 51.  A round is as wide as the kernel
+    // that runs: FP64 with the fused dval holds 16 warps an SM, not 20 (Zipf-100k
+    // k = 16: 61 us in 504-item tiles, which two rounds of 20 would have rejected, 72 in 264).
     const int small = vw == 4 ? spmm_small_tile(kk) : vw == 2 ? kDefaultItems : items;
     if (kk >= 4 && small < items && spmm_config_exists(kk, vw, small)) {
-        const int warps = spmm_warps();
-        const bool one_round = tile_rounds(p, small, warps) <= 1;
-        if ((kk >= 16 || one_round) && tile_cost(p, small, warps) < tile_cost(p, items, warps))
+        auto rounds = [&](int t) { return tile_rounds(p, kk, vw, t, o.dv_out != nullptr); };
+        auto cost = [&](int t) { return rounds(t) * (t + kTileCost); };
+        if ((kk >= 16 || rounds(small) <= 1) && cost(small) < cost(items))
             items = small;
     }
     return {kk, cols, vw, items};

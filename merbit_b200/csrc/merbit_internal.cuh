@@ -665,6 +665,9 @@ bool spmm_config_exists(int k, int vw, int items);
 int spmm_tile_candidates(int k, int* out);
 int spmm_odd_tile(int k);
 int spmm_small_tile(int k);  // the smaller of the two odd tiles
+// Warps of a configuration that a device of `sms` SMs is sure to hold (dv: with
+// the fused dval).
+int spmm_resident_warps(int dtype, int k, int vw, int items, bool dv, int sms);
 // The tile of an odd length per lane group at vector width 2, which single
 // matrices take (not among the batch's candidates; 0 if k has none).
 int spmm_odd_tile2(int k);

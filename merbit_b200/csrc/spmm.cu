@@ -438,6 +438,10 @@ __device__ __forceinline__ void drain_spmm_look_backs(const SpmmLookBack* q, int
     __syncwarp();
 }
 
+constexpr bool spmm_staged_products(int k, int vw, int items, bool dv) {
+    return k == 2 && vw == 2 && (items == 224 || items == 352) && !dv;
+}
+
 // DV: also form dL/dval for each nonzero (SpmmLaunch::dv_*), from the x row
 // the walk gathers anyway and the current row of dv_x.
 template <int DT, int K, int VW, int ITEMS, bool DV = false>
@@ -461,7 +465,7 @@ struct SpmmTile {
     // lane-contiguously, every gather in flight at once, and stores the
     // products in shared memory; each lane then walks its segment from
     // there.  The chunked walk instead keeps only CH nonzeros ahead per lane.
-    static constexpr bool STAGEP = K == 2 && VW == 2 && (ITEMS == 224 || ITEMS == 352) && !DV;
+    static constexpr bool STAGEP = spmm_staged_products(K, VW, ITEMS, DV);
     static constexpr int NJ = ITEMS / 32;  // staged products per lane
     static constexpr int CAP = ITEMS + 32;
     static constexpr int RPC = ITEMS + 16;  // row_ptr window (any rows per tile, and the
@@ -958,13 +962,13 @@ struct SpmmStage {
 // fused dval, with two tile sizes or with 8 scalar gathers ahead would spill
 // at 5; FP32 with staged products takes 6 (80 registers; an 80 x 70 x 60
 // 27-point stencil at k = 2: 80, 71, 68 and 76 us at 4, 5, 6 and 7).
-template <int DT, int K, int VW, int ITEMS, int ITEMS2, bool DV>
-constexpr int kSpmmMinCtas =
-    DT == MERBIT_F64 ? (DV || ITEMS2 != 0 || VW == 1 ? 4 : 5)
-                     : (SpmmTile<DT, K, VW, ITEMS, DV>::STAGEP ? 6 : 5);
+constexpr int spmm_ctas(int dt, int k, int vw, int items, int items2, bool dv) {
+    if (dt == MERBIT_F64) return dv || items2 != 0 || vw == 1 ? 4 : 5;
+    return spmm_staged_products(k, vw, items, dv) ? 6 : 5;
+}
 
 template <int DT, int K, int VW, int ITEMS, int ITEMS2, int WARPS, bool DV>
-__global__ void __launch_bounds__(WARPS * 32, kSpmmMinCtas<DT, K, VW, ITEMS, ITEMS2, DV>)
+__global__ void __launch_bounds__(WARPS * 32, spmm_ctas(DT, K, VW, ITEMS, ITEMS2, DV))
     spmm_kernel(const SpmmLaunch a) {
     using St = SpmmStage<DT, K, VW, ITEMS, ITEMS2, DV>;
     using T = typename St::T1;
@@ -1156,6 +1160,10 @@ bool spmm_config_exists(int k, int vw, int items) {
     case 32: return items == 260 || items == 508;
     }
     return false;
+}
+
+int spmm_resident_warps(int dtype, int k, int vw, int items, bool dv, int sms) {
+    return 4 * spmm_ctas(dtype, k, vw, items, 0, dv) * sms;
 }
 
 int spmm_tile_candidates(int k, int* out) {
