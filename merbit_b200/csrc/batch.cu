@@ -93,11 +93,12 @@ int device_sms() {
 
 // What a launch with tiles of `items` merge items takes, in items: the rounds
 // of its busiest warp, each tile costing about kTileCost items beyond its own.
+// A last round that is less than `spare` tenths full is left out.
 constexpr int kTileCost = 100;
-long long tile_rounds(const merbit_plan_s* p, int kk, int vw, int items, bool dv) {
+long long tile_rounds(const merbit_plan_s* p, int kk, int vw, int items, bool dv, int spare = 0) {
     const long long tiles = ((long long)p->nrow + p->nnz + items - 1) / items;
     const int warps = spmm_resident_warps(p->dtype, kk, vw, items, dv, device_sms());
-    return (tiles + warps - 1) / warps;
+    return std::max((tiles - (long long)warps * spare / 10 + warps - 1) / warps, 1LL);
 }
 
 // Operands of one SpMM launch: X, Y and, for a fused dval, dv_x and dv_out.
@@ -133,20 +134,28 @@ SpmmShape spmm_shape(const merbit_plan_s* p, int cols, const SpmmOperands& o) {
     int kk = 1;
     while (kk < cols) kk <<= 1;
     auto width = [&](int items) { return spmm_width(p, kk, cols, items, o); };
-    // at vector width 4 (k >= 4) the larger tiles measured faster on the
-    // power-law and banded matrices, and among them the one of an odd length
-    // per lane group (480, 496, 504, 508 items at k = 4, 8, 16, 32: no bank
-    // conflicts between the groups' segments; Zipf-1M at k = 16: 0.524 ms
-    // against 0.570 at 512); two columns as one vector take the staged products
-    // of 352-item tiles (R-MAT-300k FP32: 59 us against 70 at 256; 87 before);
-    // other shapes keep 256
+    // At vector width 4 (k >= 4) the larger tile of an odd length per lane group (480,
+    // 496, 504, 508 items at k = 4, 8, 16, 32: no bank conflicts between the groups'
+    // segments) measured faster on the power-law and banded matrices.  Two columns as
+    // one vector take the staged products of 352-item tiles (R-MAT-300k FP32: 56 us
+    // against 64 at 256), in FP64 of 224-item ones (73 us against 84 at 352 and 82 at
+    // 256; Zipf-1M 208 against 264 and 260; a 400 x 400 5-point grid 16.5 against 19
+    // and 17).  One column takes 480 items, unless 256-item tiles fill one round at
+    // most: FP32 R-MAT-300k 45 us against 53 at 256, an 80 x 70 x 60 27-point stencil 45
+    // against 56, the 5-point grid 10.2 against 12.8; R-MAT-20k 13.8 against 11.9.  With
+    // the fused dval 480 in FP64 from three rounds on (Zipf-300k 88 us against 98;
+    // R-MAT-20k, half a round, 17.9 against 18.4); not in FP32 (R-MAT-300k 98 against 91).
+    // Other shapes keep 256.
     int items = kDefaultItems;
-    if (kk >= 4 && width(512) == 4) {
-        items = 512;
-        const int odd = spmm_odd_tile(kk);
-        if (odd && width(odd) == 4) items = odd;
-    } else if (kk == 2 && !o.dv_out && width(352) == 2) {
-        items = 352;
+    const bool dv = o.dv_out != nullptr;
+    if (kk >= 4 && width(spmm_odd_tile(kk)) == 4) {
+        items = spmm_odd_tile(kk);
+    } else if (kk == 2 && !dv && width(352) == 2) {
+        items = p->dtype == MERBIT_F64 ? 224 : 352;
+    } else if (kk == 1) {
+        const bool long_enough = dv ? p->dtype == MERBIT_F64 && tile_rounds(p, 1, 1, 480, true) >= 3
+                                    : tile_rounds(p, 1, 1, 256, false) > 1;
+        if (long_enough) items = 480;
     }
     int vw = width(items);
     // Vector width 2 in tiles of an odd length per lane group: where the operands
@@ -156,7 +165,7 @@ SpmmShape spmm_shape(const merbit_plan_s* p, int cols, const SpmmOperands& o) {
     // against 190; on an 80 x 70 x 60 27-point stencil k = 8 98 against 120, k = 32
     // 209 against 250; on Zipf-300k k = 32 227 against 301.  Not at 9 to 16 columns:
     // k = 16 on Zipf-300k takes 152 us against 129.
-    if (!o.dv_out && kk >= 4 && (vw == 2 || (vw == 4 && p->dtype == MERBIT_F64 && kk != 16))) {
+    if (!dv && kk >= 4 && (vw == 2 || (vw == 4 && p->dtype == MERBIT_F64 && kk != 16))) {
         items = spmm_odd_tile2(kk);
         vw = 2;
     }
@@ -167,12 +176,13 @@ SpmmShape spmm_shape(const merbit_plan_s* p, int cols, const SpmmOperands& o) {
     // tile: 2,000 rows FP32 k = 4, 16, 32 13 / 12, 22 / 16, 32 / 20; 20,000 rows FP64
     // k = 8 28 / 21; 60,000 rows FP32 k = 32 58 / 51.  A round is as wide as the kernel
     // that runs: FP64 with the fused dval holds 16 warps an SM, not 20 (Zipf-100k
-    // k = 16: 61 us in 504-item tiles, which two rounds of 20 would have rejected, 72 in 264).
+    // k = 16: 61 us in 504-item tiles, which two rounds of 20 would have rejected, 72 in
+    // 264).  A few tiles beyond a round cost less than one (R-MAT-20k FP64 backward
+    // k = 32: 54 us with 1.01 rounds of 260 items, 65 with half a round of 508).
     const int small = vw == 4 ? spmm_small_tile(kk) : vw == 2 ? kDefaultItems : items;
     if (kk >= 4 && small < items && spmm_config_exists(kk, vw, small)) {
-        auto rounds = [&](int t) { return tile_rounds(p, kk, vw, t, o.dv_out != nullptr); };
-        auto cost = [&](int t) { return rounds(t) * (t + kTileCost); };
-        if ((kk >= 16 || rounds(small) <= 1) && cost(small) < cost(items))
+        auto cost = [&](int t) { return tile_rounds(p, kk, vw, t, dv, 1) * (t + kTileCost); };
+        if ((kk >= 16 || tile_rounds(p, kk, vw, small, dv) <= 1) && cost(small) < cost(items))
             items = small;
     }
     return {kk, cols, vw, items};

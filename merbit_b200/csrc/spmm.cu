@@ -963,7 +963,7 @@ struct SpmmStage {
 // at 5; FP32 with staged products takes 6 (80 registers; an 80 x 70 x 60
 // 27-point stencil at k = 2: 80, 71, 68 and 76 us at 4, 5, 6 and 7).
 constexpr int spmm_ctas(int dt, int k, int vw, int items, int items2, bool dv) {
-    if (dt == MERBIT_F64) return dv || items2 != 0 || vw == 1 ? 4 : 5;
+    if (dt == MERBIT_F64) return dv || items2 != 0 || (vw == 1 && k > 1) ? 4 : 5;
     return spmm_staged_products(k, vw, items, dv) ? 6 : 5;
 }
 

@@ -48,3 +48,60 @@ def test_rounds_are_as_wide_as_the_fused_backward(dtype):
     do = O.spmm_t(A.row_ptr, A.col, v, G, A.ncol)
     da = O.spmm_t(A.row_ptr, A.col, np.abs(v), np.abs(G), A.ncol)
     assert (np.abs(dX.cpu().numpy() - do) <= TOL[dtype] * np.maximum(da, 1e-300)).all()
+
+
+def _ends_at(tile, seg, items, seed):
+    """At least `items` merge items in rows that end at, before and after the ends
+    of segments and tiles; empty rows, rows over several tiles."""
+    L = np.array([seg - 1, seg, seg - 2, 0, 0, tile - 1, tile, tile - 2, 1, 2, 2 * tile - 1, 0, 3 * tile,
+                  5 * tile + 7, 1, 1, 0, 4 * seg])
+    L = np.tile(L, -(-items // int(L.sum() + L.size)))
+    rng = np.random.default_rng(seed)
+    rp = np.concatenate([[0], np.cumsum(L)]).astype(np.int32)
+    nnz, ncol = int(rp[-1]), 3000
+    return synth.CSR(rp, rng.integers(0, ncol, nnz, dtype=np.int32), rng.standard_normal(nnz), ncol, "ends")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["f64", "f32", "bf16"])
+@pytest.mark.parametrize("k, tile", [(1, 480), (2, None), (1, 256)])
+def test_one_and_two_columns_at_tile_ends(dtype, k, tile):
+    tile = tile or (224 if dtype == "f64" else 352)
+    few = tile == 256  # one round of 256-item tiles
+    A = _ends_at(tile, tile // 32, 400_000 if few else 256 * _warps(5) + 50_000, seed=k)
+    xy = np.float64 if dtype == "f64" else np.float32
+    X = synth.uniform(7, A.ncol * k).reshape(A.ncol, k).astype(xy)
+    plan = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
+    Xd = torch.from_numpy(X).cuda()
+    tiles, Y = _added_tiles(plan, lambda: plan.spmm(Xd))
+    # (480 items are FP64's and FP32's first SpMV partition: nothing is added)
+    assert tiles == (-1 if tile == 480 else -(-(A.nrow + A.nnz) // tile))
+    yo, ya = O.spmm(A.row_ptr, A.col, stored_values(A, dtype), X, k=k)
+    for _ in range(3):  # both parities
+        Y = plan.spmm(Xd, alpha=-0.5, beta=0.0)
+        e = np.abs(Y.cpu().numpy().reshape(A.nrow, k) + 0.5 * yo.reshape(A.nrow, k))
+        assert (e <= TOL[dtype] * np.maximum(ya.reshape(A.nrow, k), 1e-300)).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_one_column_fused_backward_at_tile_ends(dtype):
+    """Three rounds of 480-item tiles (FP64) on the transpose plan."""
+    B = _ends_at(480, 15, 2 * 480 * _warps(5) + 50_000, seed=3)
+    rows = np.repeat(np.arange(B.nrow, dtype=np.int32), np.diff(B.row_ptr))
+    order = np.lexsort((rows, B.col))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(B.col, minlength=B.ncol))]).astype(np.int32)
+    A = synth.CSR(rp, rows[order], B.vals[order], B.nrow, "ends transposed")
+    xy = np.float64 if dtype == "f64" else np.float32
+    G = synth.uniform(8, A.nrow).reshape(-1, 1).astype(xy)
+    X = synth.uniform(9, A.ncol).reshape(-1, 1).astype(xy)
+    M = SparseMatrix(*to_cuda(A, dtype), ncol=A.ncol)
+    dX, dv = M.backward_fused(torch.from_numpy(G).cuda(), torch.from_numpy(X).cuda())
+    v = stored_values(A, dtype)
+    do = O.spmm_t(A.row_ptr, A.col, v, G, A.ncol)
+    da = O.spmm_t(A.row_ptr, A.col, np.abs(v), np.abs(G), A.ncol)
+    assert (np.abs(dX.cpu().numpy() - do) <= TOL[dtype] * np.maximum(da, 1e-300)).all()
+    ar = np.repeat(np.arange(A.nrow), np.diff(A.row_ptr))
+    want = (G.astype(np.float64)[ar] * X.astype(np.float64)[A.col])[:, 0]
+    # one product, rounded once
+    assert (np.abs(dv.cpu().numpy() - want) <= np.finfo(xy).eps * np.abs(want)).all()
