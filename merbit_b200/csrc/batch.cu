@@ -40,21 +40,22 @@ constexpr int kBatchDefaultVariant = 6;
 
 bool pow2(int k) { return k > 0 && (k & (k - 1)) == 0; }
 
+// Whether rows of X of a type of `esz` bytes, ldx apart, can be loaded vw values
+// at a time.
+bool width_allowed(int vw, long long ldx, const void* x, long long ldy, size_t esz) {
+    if (vw == 1) return true;
+    const size_t a = vw * esz;  // vector load size
+    return ldx % vw == 0 && (uintptr_t)x % (a < 16 ? a : 16) == 0 &&
+           // the kernel keeps the distance of rows in 32 bits
+           std::max(ldx, ldy) <= (long long)(UINT_MAX / (unsigned)esz);
+}
+
 // Widest RHS vector per lane (4, 2, 1) that the leading dimension and the
 // pointers allow for k columns of a type of `esz` bytes.
-int pick_vw(int k, long long ldx, const void* x, const void* y, long long ldy, int esz,
-            int items) {
-    for (int vw = 4; vw >= 1; vw >>= 1) {
-        if (vw > k || !spmm_config_exists(k, vw, items)) continue;
-        if (vw == 1) return 1;
-        const size_t a = (size_t)vw * esz;  // vector load size
-        if (ldx % vw != 0) continue;
-        // the kernel keeps the distance of rows in 32 bits
-        if (std::max(ldx, ldy) > (long long)(UINT_MAX / (unsigned)esz)) continue;
-        if (((uintptr_t)x % (a < 16 ? a : 16)) != 0) continue;
-        (void)y;
-        return vw;
-    }
+int pick_vw(int k, long long ldx, const void* x, long long ldy, int esz, int items) {
+    for (int vw = 4; vw > 1; vw >>= 1)
+        if (vw <= k && spmm_config_exists(k, vw, items) && width_allowed(vw, ldx, x, ldy, (size_t)esz))
+            return vw;
     return 1;
 }
 
@@ -118,15 +119,18 @@ struct SpmmShape {
     int kk, cols, vw, items;
 };
 
-// Widest vector width the operands allow (with a fused dval, dv_x rows are
-// loaded with the same width).
+// Widest vector width the operands allow for a configuration (with a fused
+// dval, dv_x rows are loaded with the same width); 0 if it has none.
 int spmm_width(const merbit_plan_s* p, int kk, int cols, int items, const SpmmOperands& o) {
-    const int esz = (int)xy_size(p->dtype);
-    int vw = pick_vw(kk, o.ldx, o.x, o.y, o.ldy, esz, items);
-    while (vw > 1 && cols % vw != 0) vw >>= 1;  // a lane's columns are all used or none
-    if (o.dv_out)
-        while (vw > 1 && (o.dv_ldx % vw != 0 || (uintptr_t)o.dv_x % ((size_t)vw * esz) != 0)) vw >>= 1;
-    return vw;
+    const size_t esz = xy_size(p->dtype);
+    for (int vw = 4; vw >= 1; vw >>= 1) {
+        if (vw > kk || !spmm_single_exists(kk, vw, items)) continue;
+        if (cols % vw != 0) continue;  // a lane's columns are all used or none
+        if (!width_allowed(vw, o.ldx, o.x, o.ldy, esz)) continue;
+        if (o.dv_out && (o.dv_ldx % vw != 0 || (uintptr_t)o.dv_x % (vw * esz) != 0)) continue;
+        return vw;
+    }
+    return 0;
 }
 
 // The shape of a launch over `cols` columns.
@@ -213,6 +217,22 @@ int spmm_reserve(merbit_plan_s* p, const SpmmShape& h, cudaStream_t s, bool* roo
     }
     if (st != MERBIT_OK) *room = !out_of_memory();
     return st;
+}
+
+// A shape that the plan holds slots for and that takes the first of `left`
+// columns: all of them in the narrowest kernel that can, else as many as possible.
+bool spmm_held_shape(const merbit_plan_s* p, int left, const SpmmOperands& o, SpmmShape* out) {
+    SpmmShape best = {0, 0, 0, 0};
+    for (const auto& kv : p->spmm_slots) {  // by width, then tile
+        const int kk = (int)(kv.first >> 20), items = (int)(kv.first & ((1 << 20) - 1));
+        const int cols = std::min(left, kk);
+        if (o.dv_out && kk != left) continue;  // the dval sums run over all of the kernel's columns
+        const int vw = spmm_width(p, kk, cols, items, o);
+        if (vw && (cols > best.cols || (cols == best.cols && kk == best.kk && vw > best.vw)))
+            best = {kk, cols, vw, items};
+    }
+    *out = best;
+    return best.cols > 0;
 }
 
 // The launch, its slots reserved.
@@ -304,7 +324,7 @@ int batch_vw(const merbit_batch_s* b, int items) {
     int vw = 4;
     const int esz = (int)xy_size(b->dtype);
     for (int i = 0; i < b->count; ++i)
-        vw = std::min(vw, pick_vw(b->k, b->ldx[i], b->x[i], b->y[i], b->ldy[i], esz, items));
+        vw = std::min(vw, pick_vw(b->k, b->ldx[i], b->x[i], b->ldy[i], esz, items));
     return spmm_config_exists(b->k, vw, items) ? vw : 1;
 }
 
@@ -467,7 +487,9 @@ int merbit_spmm(merbit_plan plan, int32_t k, double alpha, const void* d_x, int6
         SpmmShape h = spmm_shape(plan, std::min(k - j, 32), o);
         bool room = true;
         int st = spmm_reserve(plan, h, s, &room);
-        if (!room && h.cols < h.kk) {  // as many columns as a narrower kernel's own
+        if (!room && spmm_held_shape(plan, h.cols, o, &h)) {
+            st = MERBIT_OK;  // slots of another width or tile
+        } else if (!room && h.cols < h.kk) {  // as many columns as a narrower kernel's own
             h = spmm_shape(plan, h.kk >> 1, o);
             st = spmm_reserve(plan, h, s, &room);
         }
@@ -493,9 +515,10 @@ int merbit_spmm_dval(merbit_plan tplan, int32_t k, const void* d_g, int64_t ldg,
         return fail(MERBIT_ERR_INVALID, "spmm_dval: null pointer");
     cudaStream_t s = (cudaStream_t)stream;
     const SpmmOperands o = {d_g, ldg, d_dx, lddx, d_x, ldx, d_dval};
-    const SpmmShape h = spmm_shape(tplan, k, o);
+    SpmmShape h = spmm_shape(tplan, k, o);
     bool room = true;
-    const int st = spmm_reserve(tplan, h, s, &room);
+    int st = spmm_reserve(tplan, h, s, &room);
+    if (!room && spmm_held_shape(tplan, k, o, &h)) st = MERBIT_OK;
     return st == MERBIT_OK ? spmm_run(tplan, h, o, 1.0, 0.0, s) : st;
 }
 

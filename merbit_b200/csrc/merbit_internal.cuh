@@ -671,6 +671,8 @@ int spmm_resident_warps(int dtype, int k, int vw, int items, bool dv, int sms);
 // The tile of an odd length per lane group at vector width 2, which single
 // matrices take (not among the batch's candidates; 0 if k has none).
 int spmm_odd_tile2(int k);
+// What a single matrix can run: spmm_config_exists and the tiles that it alone takes.
+bool spmm_single_exists(int k, int vw, int items);
 
 }  // namespace merbit
 

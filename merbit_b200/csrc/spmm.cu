@@ -808,8 +808,8 @@ struct SpmmTile {
             const int steps = __reduce_max_sync(0xFFFFFFFFu, (lx_end - lx + 2 * CH - 1) / (2 * CH));
             // The last step loads no chunk beyond it where segments are short, a few
             // steps each (k = 1: 5% less time); on longer ones the branch costs more
-            // than the load, and plain FP64 products would pass 96 registers.
-            constexpr bool kLastLoad = K >= 16 || (DT == MERBIT_F64 && !DV);
+            // than the load, and FP64 kernels would pass the registers they are bound to.
+            constexpr bool kLastLoad = K >= 16 || (DT == MERBIT_F64 && (!DV || K >= 8));
             int c = lx;
             if (steps > 0) load_chunk(c, xa, va);
             for (int i = 1; i <= steps; ++i) {
@@ -1132,16 +1132,20 @@ int launch_spmm_dt(int k, int vw, int items, int items2, const SpmmLaunch& a, cu
     // against 2.39), so k = 4 has no such tile
     MERBIT_SPMM_CASE(2, 2, 224)
     MERBIT_SPMM_CASE(2, 2, 352)
+    // odd segments at vector width 2, single matrices
+    MERBIT_SPMM_CASE(4, 2, 496)
+    MERBIT_SPMM_CASE(8, 2, 504)
+    MERBIT_SPMM_CASE(16, 2, 508)
+    MERBIT_SPMM_CASE(32, 2, 510)
+    // the same tiles at width 1: for operands that allow no more, while a capturing
+    // stream leaves the slots of these tiles only
+    MERBIT_SPMM_CASE(2, 1, 224)
+    MERBIT_SPMM_CASE(2, 1, 352)
+    MERBIT_SPMM_CASE(4, 1, 496)
+    MERBIT_SPMM_CASE(8, 1, 504)
+    MERBIT_SPMM_CASE(16, 1, 508)
+    MERBIT_SPMM_CASE(32, 1, 510)
 #undef MERBIT_SPMM_CASE
-    // odd segments at vector width 2 (single matrices without the fused dval)
-#define MERBIT_SPMM_PLAIN_CASE(KK, VV, II)                  \
-    if (k == KK && vw == VV && items == II && !a.dv_out)    \
-        return launch_spmm_cfg<DT, KK, VV, II, 4, false>(a, s);
-    MERBIT_SPMM_PLAIN_CASE(4, 2, 496)
-    MERBIT_SPMM_PLAIN_CASE(8, 2, 504)
-    MERBIT_SPMM_PLAIN_CASE(16, 2, 508)
-    MERBIT_SPMM_PLAIN_CASE(32, 2, 510)
-#undef MERBIT_SPMM_PLAIN_CASE
     return fail(MERBIT_ERR_INVALID, "spmm: no such configuration");
 }
 
@@ -1164,6 +1168,11 @@ bool spmm_config_exists(int k, int vw, int items) {
 
 int spmm_resident_warps(int dtype, int k, int vw, int items, bool dv, int sms) {
     return 4 * spmm_ctas(dtype, k, vw, items, 0, dv) * sms;
+}
+
+bool spmm_single_exists(int k, int vw, int items) {
+    if (k == 2 && vw == 1 && (items == 224 || items == 352)) return true;
+    return spmm_config_exists(k, vw, items) || (k >= 4 && vw <= 2 && items == spmm_odd_tile2(k));
 }
 
 int spmm_tile_candidates(int k, int* out) {
