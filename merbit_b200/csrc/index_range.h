@@ -11,15 +11,17 @@
 namespace merbit {
 
 // The SpMM walk counts nonzeros as in the whole matrix, and all lanes of a warp
-// take as many steps as the longest of its segments.  A lane group that is done
-// stays at the end of its own segment: what it looks ahead from there (two
-// chunks, 16 nonzeros at most) is within the 64 that the plan keeps free.
-MERBIT_HD int walk_next(int c, int by, int end) { return c + by < end ? c + by : end; }
-// nonzero c + t of a chunk; past the segment's end one of the tile again
-MERBIT_HD int walk_entry(int c, int t, int last) { return c + t < last ? c + t : last; }
+// take as many steps as the longest of its segments: the counter of a lane group
+// that is done runs up to 600 beyond the last nonzero.  It is unsigned, so that
+// it stays above every end it is compared with.
+// Nonzero c + t of a chunk; past the segment's end one of the tile again.
+MERBIT_HD int walk_entry(unsigned c, unsigned t, int last) {
+    return c + t < (unsigned)last ? (int)(c + t) : last;
+}
+// whether nonzero c + t lies in the segment
+MERBIT_HD bool walk_in(unsigned c, unsigned t, int end) { return c + t < (unsigned)end; }
 // whether no row or segment ends at or before nonzero c + n
-MERBIT_HD bool walk_clear(int lim, int c, int n) { return lim > c + n; }
-
+MERBIT_HD bool walk_clear(int lim, unsigned c, unsigned n) { return (unsigned)lim > c + n; }
 
 // f(i) for i = first, first + stride, ... below n: unsigned, as the last step
 // passes n by up to a grid's threads (1.2 million) and n may be INT_MAX (+ 1)

@@ -710,7 +710,7 @@ struct SpmmTile {
         // (past the segment's end a nonzero of the tile is read again: loads
         // without conditions; used only when the tile has nonzeros)
         const int e_last = max(lx_end - 1, x0);
-        auto load_chunk = [&](int c, XRow<X, VW> (&xr)[CH], V (&vv)[CH]) {
+        auto load_chunk = [&](unsigned c, XRow<X, VW> (&xr)[CH], V (&vv)[CH]) {
 #pragma unroll
             for (int t = 0; t < CH; ++t) {
                 const int e = walk_entry(c, t, e_last);
@@ -722,8 +722,9 @@ struct SpmmTile {
         // nonzeros c .. c + CH - 1 (those below lx_end); every row that ends at
         // or before c is finished, so c belongs to row ly.  Called by all
         // lanes of the warp.
-        auto consume = [&](int c, const XRow<X, VW> (&xr)[CH], const V (&vv)[CH]) {
-            if (__all_sync(0xFFFFFFFFu, walk_clear(lim, c, CH))) {  // no row or segment ends here
+        auto consume = [&](unsigned at, const XRow<X, VW> (&xr)[CH], const V (&vv)[CH]) {
+            const int c = (int)at;  // used below lx_end only
+            if (__all_sync(0xFFFFFFFFu, walk_clear(lim, at, CH))) {  // no row or segment ends here
                 if constexpr (CH == 2) {
                     // F32/BF16: one compensated addition of the fused pair
                     acc.add_two(to_p(vv[0]), xr[0], to_p(vv[1]), xr[1]);
@@ -741,8 +742,8 @@ struct SpmmTile {
                 return;
             }
             if constexpr (CH == 2) {
-                const bool both = lim >= c + 2;
-                if (c < lx_end) {
+                const bool both = walk_clear(lim, at, 1);
+                if (walk_in(at, 0, lx_end)) {
                     acc.add_two(to_p(vv[0]), xr[0], to_p(vv[1]), xr[1], both);
                     if (DV) {
                         dv_one(c, xr[0]);
@@ -760,7 +761,7 @@ struct SpmmTile {
             } else {
 #pragma unroll
                 for (int t = 0; t < CH; ++t) {
-                    if (c + t < lx_end) {
+                    if (walk_in(at, t, lx_end)) {
                         acc.add(to_p(vv[t]), xr[t]);
                         if (DV) dv_one(c + t, xr[t]);
                         if (next_end == c + t + 1) end_row(c + t + 1);
@@ -810,14 +811,14 @@ struct SpmmTile {
             // steps each (k = 1: 5% less time); on longer ones the branch costs more
             // than the load, and FP64 kernels would pass the registers they are bound to.
             constexpr bool kLastLoad = K >= 16 || (DT == MERBIT_F64 && (!DV || K >= 8));
-            int c = lx;
+            unsigned c = (unsigned)lx;
             if (steps > 0) load_chunk(c, xa, va);
             for (int i = 1; i <= steps; ++i) {
                 load_chunk(c + CH, xb, vb);
                 consume(c, xa, va);
                 if (kLastLoad || i < steps) load_chunk(c + 2 * CH, xa, va);  // warp-uniform
                 consume(c + CH, xb, vb);
-                c = walk_next(c, 2 * CH, lx_end);
+                c += 2 * CH;
             }
         }
 

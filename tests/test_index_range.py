@@ -30,26 +30,27 @@ static int walk(int nrow, int nnz, int seg, int groups, int ch, int L) {
         for (int g = 0; g < groups; ++g) {
             const int lx = at(g), end = at(g + 1);
             const int last = std::max(end - 1, x0);
-            int c = lx, taken = 0;
-            auto load = [&](int from) {
+            unsigned c = (unsigned)lx;
+            int taken = 0;
+            auto load = [&](unsigned from) {
                 for (int t = 0; t < ch; ++t) {
                     const int e = walk_entry(from, t, last);
                     if (e < x0 || e >= std::max(x1, x0 + 1)) return false;
                 }
                 return true;
             };
-            auto consume = [&](int from) {
+            auto consume = [&](unsigned from) {
                 if (walk_clear(end, from, ch)) {
                     taken += ch;
                 } else {
-                    for (int t = 0; t < ch; ++t) taken += from + t < end;
+                    for (int t = 0; t < ch; ++t) taken += walk_in(from, t, end);
                 }
             };
             for (int i = 0; i < steps; ++i) {
                 if (!load(c) || !load(c + ch) || !load(c + 2 * ch)) return 1;
                 consume(c);
                 consume(c + ch);
-                c = walk_next(c, 2 * ch, end);
+                c += 2 * ch;
             }
             if (taken != end - lx) return 2;
         }
