@@ -94,12 +94,11 @@ int device_sms() {
 
 // What a launch with tiles of `items` merge items takes, in items: the rounds
 // of its busiest warp, each tile costing about kTileCost items beyond its own.
-// A last round that is less than `spare` tenths full is left out.
 constexpr int kTileCost = 100;
-long long tile_rounds(const merbit_plan_s* p, int kk, int vw, int items, bool dv, int spare = 0) {
+long long tile_rounds(const merbit_plan_s* p, int kk, int vw, int items, bool dv) {
     const long long tiles = ((long long)p->nrow + p->nnz + items - 1) / items;
     const int warps = spmm_resident_warps(p->dtype, kk, vw, items, dv, device_sms());
-    return std::max((tiles - (long long)warps * spare / 10 + warps - 1) / warps, 1LL);
+    return (tiles + warps - 1) / warps;
 }
 
 // Operands of one SpMM launch: X, Y and, for a fused dval, dv_x and dv_out.
@@ -185,8 +184,11 @@ SpmmShape spmm_shape(const merbit_plan_s* p, int cols, const SpmmOperands& o) {
     // k = 32: 54 us with 1.01 rounds of 260 items, 65 with half a round of 508).
     const int small = vw == 4 ? spmm_small_tile(kk) : vw == 2 ? kDefaultItems : items;
     if (kk >= 4 && small < items && spmm_config_exists(kk, vw, small)) {
-        auto cost = [&](int t) { return tile_rounds(p, kk, vw, t, dv, 1) * (t + kTileCost); };
-        if ((kk >= 16 || tile_rounds(p, kk, vw, small, dv) <= 1) && cost(small) < cost(items))
+        auto cost = [&](int t) { return tile_rounds(p, kk, vw, t, dv) * (t + kTileCost); };
+        // one round and a tenth of a round count as one
+        const bool few = tile_rounds(p, kk, vw, small + small / 10, dv) <= 1;
+        if (kk >= 16 ? few || cost(small) < cost(items)
+                     : tile_rounds(p, kk, vw, small, dv) <= 1 && cost(small) < cost(items))
             items = small;
     }
     return {kk, cols, vw, items};
