@@ -194,6 +194,47 @@ SpmmShape spmm_shape(const merbit_plan_s* p, int cols, const SpmmOperands& o) {
     return {kk, cols, vw, items};
 }
 
+// Columns of the next launch when `left` are left: at most 32, and without the
+// last one where it would make the others slow: one column more than a multiple
+// of 4 leaves every lane scalar loads, and after 8 or 16 it doubles the kernel's
+// width as well.  Measured whole / with the last column in a launch of its own (us;
+// R-MAT-300k, 80 x 70 x 60 27-point stencil, 150,000 rows of 0 to 40):
+//   FP32, rows of X on 16 bytes   k =  9  175 / 133   217 / 145    90 / 77
+//                                 k = 17  251 / 160   309 / 175   131 / 92
+//                                 k = 21  252 / 198   309 / 240   131 / 113
+//                                 k =  5  135 / 116   148 / 132    62 / 70
+//   FP32, rows on 8 bytes         k = 17  251 / 168   309 / 193   131 / 94
+//   FP32, rows on 4 bytes         k = 17  252 / 222   309 / 266   131 / 117
+//                                 k =  9  175 / 182   217 / 193    89 / 89
+//   FP64, rows on 16 bytes        k = 17  231 / 192   294 / 233   118 / 98
+//                                 k =  9  165 / 162   205 / 172    83 / 85
+//                                 k = 21  232 / 264   295 / 317   118 / 131
+// A small matrix is better read once: below 2 million items (R-MAT-20k FP32 k = 21
+// 37 / 40), for 9 and 17 columns in whole vectors below 700,000, and where the gain
+// is least (5 columns, 9 in FP64) below 4 million.
+int spmm_columns(const merbit_plan_s* p, int left, const SpmmOperands& o) {
+    const int cols = std::min(left, 32);
+    if (cols % 4 != 1 || cols == 1) return cols;
+    const size_t esz = xy_size(p->dtype);
+    const int w = width_allowed(4, o.ldx, o.x, o.ldy, esz) ? 4 : width_allowed(2, o.ldx, o.x, o.ldy, esz) ? 2 : 1;
+    const long long items = (long long)p->nrow + p->nnz;
+    const bool doubled = cols == 9 || cols == 17;
+    long long above = 2'000'000;  // items
+    bool split;
+    if (p->dtype == MERBIT_F64) {
+        split = doubled && w >= 2;
+        if (cols == 9) above = 4'000'000;
+    } else if (w == 4) {
+        split = true;
+        if (doubled) above = 700'000;
+        if (cols == 5) above = 4'000'000;
+    } else {
+        split = cols == 17 || (cols == 9 && (w == 2 || p->dtype == MERBIT_BF16));
+    }
+    split = split && items > above;
+    return split ? cols - 1 : cols;
+}
+
 long long slot_key(const SpmmShape& h) { return ((long long)h.kk << 20) | h.items; }
 
 // Makes the partition and the carry slots of a shape when the plan has none.
@@ -478,15 +519,15 @@ int merbit_spmm(merbit_plan plan, int32_t k, double alpha, const void* d_x, int6
     cudaStream_t s = (cudaStream_t)stream;
     const size_t esz = xy_size(plan->dtype);
     // Column blocks of 32; the rest in one launch of the smallest kernel that
-    // holds it, its lanes beyond the last column idle.  One launch per power of
-    // two read the matrix up to five times: R-MAT-300k (7.2 M nonzeros) FP32
-    // took 217, 512, 294 and 765 us at k = 12, 15, 20 and 31, and takes 113,
-    // 175, 153 and 252; no k from 2 to 40 is faster split.
+    // holds it, its lanes beyond the last column idle (or less one: spmm_columns).  A
+    // launch per power of two reads the matrix up to five times: R-MAT-300k FP32
+    // k = 12, 15, 20 and 31 109, 175, 147 and 252 us, in separate launches 147, 367,
+    // 173 and 544.
     int j = 0;
     while (j < k) {
         const SpmmOperands o = {static_cast<const char*>(d_x) + (size_t)j * esz, ldx,
                                 static_cast<char*>(d_y) + (size_t)j * esz, ldy, nullptr, 0, nullptr};
-        SpmmShape h = spmm_shape(plan, std::min(k - j, 32), o);
+        SpmmShape h = spmm_shape(plan, spmm_columns(plan, k - j, o), o);
         bool room = true;
         int st = spmm_reserve(plan, h, s, &room);
         if (!room && spmm_held_shape(plan, h.cols, o, &h)) {

@@ -105,3 +105,44 @@ def test_one_column_fused_backward_at_tile_ends(dtype):
     want = (G.astype(np.float64)[ar] * X.astype(np.float64)[A.col])[:, 0]
     # one product, rounded once
     assert (np.abs(dv.cpu().numpy() - want) <= np.finfo(xy).eps * np.abs(want)).all()
+
+
+def _launches(call):
+    """Kernels that a call captures."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g, stream=s):
+        call(s)
+    err, _, n = rt.cudaGraphGetNodes(rt.cudaGraph_t(g.raw_cuda_graph()), 0)
+    assert int(err) == 0
+    return n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype, k, ld, launches", [
+    ("f32", 17, 20, 2), ("f32", 17, 17, 2), ("f32", 9, 12, 2), ("f32", 9, 10, 2), ("f32", 9, 9, 1),
+    ("f32", 21, 24, 2), ("f32", 21, 22, 1), ("f32", 49, 52, 3), ("f32", 5, 8, 1), ("f32", 20, 20, 1),
+    ("bf16", 9, 9, 2), ("bf16", 13, 16, 2), ("bf16", 17, 18, 2), ("bf16", 25, 25, 1),
+    ("f64", 17, 18, 2), ("f64", 17, 17, 1), ("f64", 21, 24, 1), ("f64", 9, 10, 1),
+])
+def test_a_last_column_of_its_own(dtype, k, ld, launches):
+    """A column more than a multiple of 4: apart where the others then take whole
+    vectors; columns beyond k are neither read nor written."""
+    A = _ends_at(504, 63, 2_050_000, seed=9)
+    xy = np.float64 if dtype == "f64" else np.float32
+    X = synth.uniform(10, A.ncol * k).reshape(A.ncol, k).astype(xy)
+    Xd = torch.full((A.ncol, ld), float("nan"), dtype=torch.from_numpy(X).dtype, device="cuda")
+    Xd[:, :k] = torch.from_numpy(X)
+    Yd = torch.full((A.nrow, ld), -7.0, dtype=Xd.dtype, device="cuda")
+    plan = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
+    yo, ya = O.spmm(A.row_ptr, A.col, stored_values(A, dtype), X, k=k)
+    for _ in range(3):
+        Yd[:, :k] = float("nan")
+        plan.spmm(Xd[:, :k], Yd[:, :k])
+        torch.cuda.synchronize()
+        e = np.abs(Yd[:, :k].cpu().numpy() - yo)
+        assert (e <= TOL[dtype] * np.maximum(ya, 1e-300)).all()
+        assert bool((Yd[:, k:] == -7.0).all())
+    assert _launches(lambda s: plan.spmm(Xd[:, :k], Yd[:, :k], stream=s)) == launches
