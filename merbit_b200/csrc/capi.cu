@@ -158,12 +158,32 @@ int plan_config_ok(merbit_plan_s* p, int idx, bool* ok, cudaStream_t s) {
 // us at one lane and 65 at 4, of 16 135 and 90; of 32 95 at 4 lanes and 93 at 8, of
 // 64 85 and 72 (FP64).  Above 128 entries a row the rule leaves the matrix to
 // the merge path, which balances any rows.
+// A group of lanes waits for the longest row of its warp.  Where the longest is
+// more than 2.5 times the mean, that is made up for only while the merge path's
+// tiles do not fill the device: skew (longest / mean) times rows up to 4.2 million,
+// twice that for 4-byte x when a row fills its 4 lanes (mean 3.75).  Row groups /
+// merge path, us, FP64 and FP32 (rows of a, a fraction f of b):
+//   rows       a, b, f           skew  FP64          FP32
+//   2,000,000  3, 40, 0.01       11.9   66 /  65      64 /  51   not taken
+//   2,000,000  0, 128, 0.1       10.0  201 / 164     193 / 148   not taken
+//   500,000    3, 128, 0.01      30.0   31 /  25      26 /  29   not taken
+//   500,000    6, 128, 0.02      15.2   39 /  35      31 /  40   FP32 alone
+//   500,000    10, 128, 0.05      8.1   59 /  60      48 /  50   taken
+//   200,000    2, 64, 0.03       16.7   12 /  13      11 /  13   taken
+//   60,000     3, 128, 0.01      29.7   11 /  11       7 /  11   taken
+// (Arrays off 16 bytes go to CTA tiles otherwise, which lose more.)
 constexpr int kShortRows = 128;
 int short_rows_choice(const merbit_plan_s* p) {
     if (p->max_row_len < 1 || p->max_row_len > kShortRows) return -1;
-    const double mean = (double)p->nnz / (double)std::max(p->nrow, 1);
+    const double rows = (double)std::max(p->nrow, 1);
+    const double mean = (double)p->nnz / rows;
     if (mean < 2.5) return -1;
     const bool lane_per_row = mean < 14.0 && p->max_row_len <= 32;
+    if (!lane_per_row && p->vec) {
+        const double skew = (double)p->max_row_len / mean;
+        const double most = p->dtype != MERBIT_F64 && mean >= 3.75 ? 8.5e6 : 4.2e6;
+        if (skew > 2.5 && skew * rows > most) return -1;
+    }
     const int lanes = lane_per_row ? 1 : mean < 40.0 ? 4 : 8;
     for (int i = 0, n = spmv_num_configs(p->dtype); i < n; ++i) {
         const SpmvConfig c = spmv_config(p->dtype, i);
@@ -177,22 +197,19 @@ int short_rows_choice(const merbit_plan_s* p) {
 // in R-MAT graphs), the first whose window holds a tile of row ends.
 int plan_pick_default(merbit_plan_s* p, cudaStream_t s) {
     const int n = spmv_num_configs(p->dtype);
-    std::vector<int> order;
     for (int pass = 0; pass < 2; ++pass)
         for (int i = 0; i < n; ++i) {
             const SpmvConfig c = spmv_config(p->dtype, i);
             const bool early = i == 0 || (c.kind == 1 && c.stg);
-            if (early == (pass == 0)) order.push_back(i);
+            if (early != (pass == 0)) continue;
+            bool ok = false;
+            int st = plan_config_ok(p, i, &ok, s);
+            if (st != MERBIT_OK) return st;
+            if (ok) {
+                p->cfg = i;
+                return MERBIT_OK;
+            }
         }
-    for (int i : order) {
-        bool ok = false;
-        int st = plan_config_ok(p, i, &ok, s);
-        if (st != MERBIT_OK) return st;
-        if (ok) {
-            p->cfg = i;
-            return MERBIT_OK;
-        }
-    }
     return fail(MERBIT_ERR_UNSUPPORTED, "no SpMV configuration fits this matrix");
 }
 
