@@ -27,22 +27,25 @@ int grid_of(long long n) {
 }
 
 __global__ void pack_keys(const int* __restrict__ major, const int* __restrict__ minor, int n,
-                          unsigned long long* __restrict__ key, int* __restrict__ idx) {
+                          int b_minor, unsigned long long* __restrict__ key,
+                          int* __restrict__ idx) {
     each_index((unsigned)n, [&](int i) {
-        key[i] = ((unsigned long long)(unsigned)major[i] << 32) | (unsigned)minor[i];
+        key[i] = ((unsigned long long)(unsigned)major[i] << b_minor) | (unsigned)minor[i];
         idx[i] = i;
     });
 }
 
-__global__ void unpack_keys(const unsigned long long* __restrict__ key, int n,
+__global__ void unpack_keys(const unsigned long long* __restrict__ key, int n, int b_minor,
                             int* __restrict__ major, int* __restrict__ minor) {
+    const unsigned long long min_mask = (1ull << b_minor) - 1;
     each_index((unsigned)n, [&](int i) {
-        major[i] = (int)(key[i] >> 32);
-        minor[i] = (int)(key[i] & 0xFFFFFFFFull);
+        major[i] = (int)(key[i] >> b_minor);
+        minor[i] = (int)(key[i] & min_mask);
     });
 }
 
-// Largest index of each array, as unsigned values.
+// Largest index of each array, as unsigned values.  One atomic per block: one per
+// warp, 76,000 on two words, took most of this kernel's time.
 __global__ void max_indices(const int* __restrict__ major, const int* __restrict__ minor, int n,
                             unsigned* __restrict__ out) {
     unsigned a = 0u, b = 0u;
@@ -50,12 +53,17 @@ __global__ void max_indices(const int* __restrict__ major, const int* __restrict
         a = max(a, (unsigned)major[i]);
         b = max(b, (unsigned)minor[i]);
     });
+    __shared__ unsigned top[2];
+    if (threadIdx.x < 2) top[threadIdx.x] = 0u;
+    __syncthreads();
     a = __reduce_max_sync(0xFFFFFFFFu, a);
     b = __reduce_max_sync(0xFFFFFFFFu, b);
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(out, a);
-        atomicMax(out + 1, b);
+        atomicMax(top, a);
+        atomicMax(top + 1, b);
     }
+    __syncthreads();
+    if (threadIdx.x < 2) atomicMax(out + threadIdx.x, top[threadIdx.x]);
 }
 
 // One word per triplet: major, minor (b_minor bits) and position (b_pos bits).
@@ -134,7 +142,6 @@ int merbit_coo_sort(int32_t nnz, int32_t* d_major, int32_t* d_minor, void* d_val
     cudaStream_t s = (cudaStream_t)stream;
     unsigned long long *k_in = nullptr, *k_out = nullptr;
     int *i_in = nullptr, *i_out = nullptr;
-    void* tmpv = nullptr;
     void* temp = nullptr;
     const size_t vs = dtype_size(dtype);
     auto done = [&](int st) {  // stream-ordered: after the sort's own work on s
@@ -142,7 +149,6 @@ int merbit_coo_sort(int32_t nnz, int32_t* d_major, int32_t* d_minor, void* d_val
         dev_free(k_out, s);
         dev_free(i_in, s);
         dev_free(i_out, s);
-        dev_free(tmpv, s);
         dev_free(temp, s);
         return st;
     };
@@ -160,8 +166,10 @@ int merbit_coo_sort(int32_t nnz, int32_t* d_major, int32_t* d_minor, void* d_val
     // keys alone are sorted, over b1 + b2 bits, between two buffers, and the
     // buffer that is free afterwards takes the values.  4 M triplets of a 250,000
     // node graph: 5 passes over 8 bytes instead of 8 over 12 (0.19 ms instead of
-    // 0.42), and 64 MB of work space instead of 180, which the pool can keep
-    // (it unmapped the rest at every call: 2 to 13 ms).
+    // 0.42), and 64 MB of work space instead of 144.  That is what the pool keeps
+    // mapped when nothing else is alive: the whole call takes 0.38 ms.  From 4.2 M
+    // triplets on, or with other blocks alive, part of it is unmapped and mapped again at
+    // every call (0.8 ms; 8 M 1.5 ms; 4 M beside a plan and its transpose 1.2 ms).
     TRY_ALLOC(k_in, 8 * (size_t)nnz);
     TRY_ALLOC(k_out, 8 * (size_t)nnz);
     unsigned top[2] = {0u, 0u};
@@ -198,17 +206,20 @@ int merbit_coo_sort(int32_t nnz, int32_t* d_major, int32_t* d_minor, void* d_val
         TRY(cudaStreamSynchronize(s));
         return done(MERBIT_OK);
     }
-    // wider indices (or negative ones, as unsigned): 64-bit keys and positions
+    // wider indices (or negative ones, as unsigned): keys and positions apart, sorted
+    // over the bits that the indices use: two passes fewer than over 64 bits make up
+    // for reading the largest indices back (1 M triplets of 20 million nodes 0.25 ms)
     TRY_ALLOC(i_in, 4 * (size_t)nnz);
     TRY_ALLOC(i_out, 4 * (size_t)nnz);
-    pack_keys<<<grid_of(nnz), 256, 0, s>>>(d_major, d_minor, nnz, k_in, i_in);
+    pack_keys<<<grid_of(nnz), 256, 0, s>>>(d_major, d_minor, nnz, b_minor, k_in, i_in);
     size_t tb = 0;
-    TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, k_in, k_out, i_in, i_out, nnz, 0, 64, s));
+    const int b_key = b_all - b_pos;
+    TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, k_in, k_out, i_in, i_out, nnz, 0, b_key, s));
     TRY_ALLOC(temp, tb);
-    TRY(cub::DeviceRadixSort::SortPairs(temp, tb, k_in, k_out, i_in, i_out, nnz, 0, 64, s));
-    unpack_keys<<<grid_of(nnz), 256, 0, s>>>(k_out, nnz, d_major, d_minor);
+    TRY(cub::DeviceRadixSort::SortPairs(temp, tb, k_in, k_out, i_in, i_out, nnz, 0, b_key, s));
+    unpack_keys<<<grid_of(nnz), 256, 0, s>>>(k_out, nnz, b_minor, d_major, d_minor);
     if (d_vals) {
-        TRY_ALLOC(tmpv, vs * (size_t)nnz);
+        void* tmpv = k_in;  // free after the sort
         TRY(cudaMemcpyAsync(tmpv, d_vals, vs * (size_t)nnz, cudaMemcpyDeviceToDevice, s));
         if (dtype == MERBIT_F64)
             permute_vals<double><<<grid_of(nnz), 256, 0, s>>>((const double*)tmpv, i_out, nnz,
