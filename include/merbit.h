@@ -222,9 +222,11 @@ int merbit_spmm_dval(merbit_plan tplan, int32_t k, const void* d_g, int64_t ldg,
 
 /* Y[nrow x k] = alpha*A*X[ncol x k] + beta*Y, row-major with leading
  * dimensions ldx, ldy >= k (elements).  Any k >= 1 (processed in
- * column blocks of 32, the last one narrower).  The first call for a given
- * block width allocates that width's carry slots (synchronizes); later
- * calls allocate nothing and can be captured in a CUDA graph. */
+ * column blocks of 32, the last one narrower).  The first call of a shape
+ * (k, leading dimensions, alignment) allocates carry slots and builds a
+ * partition (synchronizes); the same call then allocates nothing and can be
+ * captured in a CUDA graph.  Another shape is captured with the slots that the
+ * plan holds where they serve it, else refused with MERBIT_ERR_INVALID. */
 int merbit_spmm(merbit_plan plan, int32_t k, double alpha, const void* d_x, int64_t ldx,
                 double beta, void* d_y, int64_t ldy, void* stream);
 
@@ -254,7 +256,10 @@ typedef struct merbit_batch_info {
  * warp-tile kernel (variant 6, or the cached choices of the members'
  * signatures), at k = 2 352-item staged-product tiles, at k >= 4 the odd
  * tile of k at vector width 4 (where the operands allow them).
- * Synchronizes. */
+ * Synchronizes.  merbit_batch_tune, merbit_batch_set_kernel and the
+ * set_matrix calls below replace the batch's descriptors and carry slots in
+ * place: they wait for its launches, and a CUDA graph captured before has to
+ * be captured again. */
 int merbit_batch_create(merbit_batch* batch, int32_t count, const merbit_plan* plans, int32_t k,
                         const void* const* d_x, const int64_t* ldx, void* const* d_y,
                         const int64_t* ldy, void* stream);

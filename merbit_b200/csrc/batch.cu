@@ -340,11 +340,12 @@ int batch_upload(merbit_batch_s* b, const std::vector<SpmmDesc>& h, long long to
     if (b->d_descs == nullptr) {
         int st = dev_alloc(&b->d_descs, sizeof(SpmmDesc) * b->count, s);
         if (st != MERBIT_OK) return st;
+    } else {  // launches on any stream may use the descriptors and the slots
+        MERBIT_CUDA(cudaDeviceSynchronize());
     }
     MERBIT_CUDA(cudaMemcpyAsync(b->d_descs, h.data(), sizeof(SpmmDesc) * b->count,
                                 cudaMemcpyHostToDevice, s));
     if (b->slots.nslots < tot * b->k) {
-        if (b->slots.words) MERBIT_CUDA(cudaDeviceSynchronize());  // launches may use them
         dev_free(b->slots.words, s);
         dev_free(b->slots.state, s);
         b->slots = SpmmSlots();
@@ -353,7 +354,6 @@ int batch_upload(merbit_batch_s* b, const std::vector<SpmmDesc>& h, long long to
     } else {
         // other tiles than before: every word empty again (a launch of the
         // SpMM kernel empties only the words it uses)
-        MERBIT_CUDA(cudaDeviceSynchronize());  // launches may use them
         MERBIT_CUDA(cudaMemsetAsync(b->slots.words, 0xFF,
                                     sizeof(unsigned long long) * 4 * (size_t)b->slots.nslots, s));
     }
