@@ -145,10 +145,12 @@ __device__ __forceinline__ void finish_launch(LaunchState* st, unsigned epoch) {
 // Carry slots.  Two arrays of nslots 8-byte words, selected by the parity of
 // the launch epoch.  A tile publishes its trailing partial sum as one word in
 // the current array; a reader spins until the word is no longer kEmpty, so
-// one load returns both "ready" and the value.  Every launch refills the
-// other array with kEmpty, which makes it ready for the next launch whatever
-// tiles this one used (CUDA-graph replays included).  A value whose bits
-// happen to equal kEmpty (a NaN) is published as the canonical NaN.
+// one load returns both "ready" and the value.  Every SpMV launch, and every
+// batch launch at k = 1, refills the other array with kEmpty, which makes it ready
+// for the next launch whatever tiles this one used (CUDA-graph replays
+// included); SpMM launches empty the words that they use, which are the same for
+// every launch on the same tiles.  A value whose bits happen to equal kEmpty (a
+// NaN) is published as the canonical NaN.
 // ---------------------------------------------------------------------------
 constexpr unsigned long long kEmpty = ~0ull;
 
@@ -439,7 +441,6 @@ struct SpmvConfig {
     int kind;  // 0: CTA-tile kernel, 1: warp-tile kernel
     int block;
     int ipt;
-    int stages;  // warp-tile kernel: shared-memory stages per warp (1)
     // Warp-tile kernel: preferred shared-memory carveout in percent (0: the
     // driver's choice, which for these kernels is all shared memory).  The
     // x gathers need L1 capacity for their misses in flight; giving L1 more

@@ -26,9 +26,9 @@
 // without passing through double when alpha = 1 and beta = 0, and only the
 // slots that a launch uses are emptied for the next one (all of them, they
 // were 20 MB of L2 for Zipf-1M at k = 16, whose X of 64 MB then no longer fit).
-// Measured on B200, before and after: Zipf-1M FP32 k = 16 526 -> 351 us, its
-// fused backward 628 -> 537; Zipf-500k FP64 k = 8 210 -> 153; 32 R-MAT
-// matrices FP32 in one launch, k = 4 603 -> 435, k = 32 1,540 -> 1,070.
+// Measured on B200 (one launch of a CUDA graph): Zipf-1M FP32 k = 16 351 us, its
+// fused backward 537; Zipf-500k FP64 k = 8 153; 32 R-MAT matrices FP32 in one
+// launch, k = 4 435 us, k = 32 1,070.
 //
 // Batches: the tiles of all matrices form one index space; matrix m owns
 // tiles [tile_begin_m, tile_begin_m + num_tiles_m).  Warps of the
@@ -263,8 +263,8 @@ struct AccRow {
 // packed f32x2 instruction.  The steps are Knuth's, with n = s - t in the
 // place of -(t - s): t = s + q, e = (s - (t + n)) + (q + n).  A lone product
 // enters with its own rounding error (a x + n instead of q + n); two products
-// of one row enter as their fused sum, whose rounding is one unit of
-// |a0 x0| + |a1 x1|.
+// of one row enter as q = fma(a1, x1, a0 x0), whose two roundings cost at most
+// u (2 |a0 x0| + |a1 x1|), u = 2^-24 (half a unit in the last place).
 template <int VW>
 struct AccRow<AccTwoSum, VW, float, float> {
     static_assert(VW % 2 == 0, "packed TwoSum needs an even width");

@@ -259,51 +259,49 @@ namespace {
 // Items per thread are odd: a lane's segment then starts an odd number of
 // elements after its neighbour's, which spreads the lanes of a warp over
 // all shared-memory banks when they walk their segments in step.
-// stages: shared-memory stages per warp of the warp-tile kernel (the kernel
-// also runs 2, which measured slower: less occupancy and less L1).
 // Order matters only for the default pick (the first usable entry): the
 // large-L1 warp-tile entries come first because they are the better choice
 // for irregular matrices; plan_tune picks per matrix.
 constexpr SpmvConfig kCfgF64[] = {
-    {1, 256, 15, 1, kCarveoutL1, 1}, {1, 128, 15, 1, kCarveoutL1, 1},
-    {1, 256, 11, 1, kCarveoutL1, 1}, {1, 128, 15, 1, kCarveoutL1Max, 1},
-    {1, 256, 15, 1, kCarveoutL1, 0}, {1, 256, 15, 1, 0, 0},
-    {1, 128, 15, 1, 0, 0},           {1, 256, 11, 1, 0, 0},
-    {1, 256, 7, 1, 0, 0},            {1, 128, 23, 1, 0, 0},
-    {0, 256, 7, 1, 0, 0},            {0, 256, 11, 1, 0, 0},
-    {0, 128, 9, 1, 0, 0},
-    {3, 256, 4, 1, 0, 0},            {3, 256, 8, 1, 0, 0},
-    {3, 256, 16, 1, 0, 0},           {3, 256, 32, 1, 0, 0},
-    {3, 256, 8, 1, 0, 1},            {3, 256, 16, 1, 0, 1},
-    {3, 256, 2, 1, 0, 0},            {3, 256, 4, 1, 0, 0, 1},
-    {3, 256, 2, 1, 0, 0, 1},         {3, 256, 8, 1, 0, 0, 1},
-    {3, 256, 1, 1, 0, 0, 1},
+    {1, 256, 15, kCarveoutL1, 1}, {1, 128, 15, kCarveoutL1, 1},
+    {1, 256, 11, kCarveoutL1, 1}, {1, 128, 15, kCarveoutL1Max, 1},
+    {1, 256, 15, kCarveoutL1, 0}, {1, 256, 15, 0, 0},
+    {1, 128, 15, 0, 0},           {1, 256, 11, 0, 0},
+    {1, 256, 7, 0, 0},            {1, 128, 23, 0, 0},
+    {0, 256, 7, 0, 0},            {0, 256, 11, 0, 0},
+    {0, 128, 9, 0, 0},
+    {3, 256, 4, 0, 0},            {3, 256, 8, 0, 0},
+    {3, 256, 16, 0, 0},           {3, 256, 32, 0, 0},
+    {3, 256, 8, 0, 1},            {3, 256, 16, 0, 1},
+    {3, 256, 2, 0, 0},            {3, 256, 4, 0, 0, 1},
+    {3, 256, 2, 0, 0, 1},         {3, 256, 8, 0, 0, 1},
+    {3, 256, 1, 0, 0, 1},
     // warp tiles added later (appended, so earlier indices stay): 13 items
     // per lane (4 CTAs of 8 warps at the 72% carveout in FP64), and tiles
     // with a row_ptr window for every item (stg = 1: no rows-per-tile cap),
     // with L1 gathers at a 58% carveout for matrices whose columns repeat
-    {1, 256, 13, 1, kCarveoutL1, 1},  {1, 256, 11, 1, kCarveoutL1Max, 0, 1},
-    {1, 256, 15, 1, kCarveoutL1Max, 0, 1}, {1, 256, 11, 1, kCarveoutL1, 1, 1}};
+    {1, 256, 13, kCarveoutL1, 1},  {1, 256, 11, kCarveoutL1Max, 0, 1},
+    {1, 256, 15, kCarveoutL1Max, 0, 1}, {1, 256, 11, kCarveoutL1, 1, 1}};
 constexpr SpmvConfig kCfgF32[] = {
-    {1, 256, 15, 1, kCarveoutL1, 1}, {1, 128, 15, 1, kCarveoutL1, 1},
-    {1, 256, 11, 1, kCarveoutL1, 1}, {1, 128, 15, 1, kCarveoutL1Max, 1},
-    {1, 256, 15, 1, kCarveoutL1, 0}, {1, 256, 15, 1, 0, 0},
-    {1, 128, 15, 1, 0, 0},           {1, 256, 11, 1, 0, 0},
-    {1, 256, 7, 1, 0, 0},            {1, 128, 23, 1, 0, 0},
-    {0, 256, 11, 1, 0, 0},           {0, 256, 7, 1, 0, 0},
-    {0, 256, 15, 1, 0, 0},
-    {3, 256, 4, 1, 0, 0},            {3, 256, 8, 1, 0, 0},
-    {3, 256, 16, 1, 0, 0},           {3, 256, 32, 1, 0, 0},
-    {3, 256, 8, 1, 0, 1},            {3, 256, 16, 1, 0, 1},
-    {3, 256, 2, 1, 0, 0},            {3, 256, 4, 1, 0, 0, 1},
-    {3, 256, 2, 1, 0, 0, 1},         {3, 256, 8, 1, 0, 0, 1},
-    {3, 256, 1, 1, 0, 0, 1},
+    {1, 256, 15, kCarveoutL1, 1}, {1, 128, 15, kCarveoutL1, 1},
+    {1, 256, 11, kCarveoutL1, 1}, {1, 128, 15, kCarveoutL1Max, 1},
+    {1, 256, 15, kCarveoutL1, 0}, {1, 256, 15, 0, 0},
+    {1, 128, 15, 0, 0},           {1, 256, 11, 0, 0},
+    {1, 256, 7, 0, 0},            {1, 128, 23, 0, 0},
+    {0, 256, 11, 0, 0},           {0, 256, 7, 0, 0},
+    {0, 256, 15, 0, 0},
+    {3, 256, 4, 0, 0},            {3, 256, 8, 0, 0},
+    {3, 256, 16, 0, 0},           {3, 256, 32, 0, 0},
+    {3, 256, 8, 0, 1},            {3, 256, 16, 0, 1},
+    {3, 256, 2, 0, 0},            {3, 256, 4, 0, 0, 1},
+    {3, 256, 2, 0, 0, 1},         {3, 256, 8, 0, 0, 1},
+    {3, 256, 1, 0, 0, 1},
     // warp tiles added later (appended, so earlier indices stay): 13 items
     // per lane (4 CTAs of 8 warps at the 72% carveout in FP64), and tiles
     // with a row_ptr window for every item (stg = 1: no rows-per-tile cap),
     // with L1 gathers at a 58% carveout for matrices whose columns repeat
-    {1, 256, 13, 1, kCarveoutL1, 1},  {1, 256, 11, 1, kCarveoutL1Max, 0, 1},
-    {1, 256, 15, 1, kCarveoutL1Max, 0, 1}, {1, 256, 11, 1, kCarveoutL1, 1, 1}};
+    {1, 256, 13, kCarveoutL1, 1},  {1, 256, 11, kCarveoutL1Max, 0, 1},
+    {1, 256, 15, kCarveoutL1Max, 0, 1}, {1, 256, 11, kCarveoutL1, 1, 1}};
 
 template <int DT, int BLOCK, int IPT, bool VEC, bool RES>
 int launch_one_k(const SpmvLaunch& a, cudaStream_t s) {

@@ -223,7 +223,6 @@ int launch_warp(const SpmvLaunch& a, cudaStream_t s) {
 template <int DT>
 int launch_warp_dt(const SpmvConfig& c, const SpmvLaunch& a, cudaStream_t s) {
     const int warps = c.block / 32, ipt = c.ipt;
-    if (c.stages != 1) return fail(MERBIT_ERR_INVALID, "spmv_warp: no such configuration");
 #define MERBIT_WARP_CASE(W, I, G, C)                                                   \
     if (warps == W && ipt == I && c.cg == G && c.carveout == C && !c.stg)              \
         return launch_warp<DT, W, I, G, C>(a, s);

@@ -74,8 +74,8 @@ def test_one_and_two_columns_at_tile_ends(dtype, k, tile):
     plan = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
     Xd = torch.from_numpy(X).cuda()
     tiles, Y = _added_tiles(plan, lambda: plan.spmm(Xd))
-    # (480 items are FP64's and FP32's first SpMV partition: nothing is added)
-    assert tiles == (-1 if tile == 480 else -(-(A.nrow + A.nnz) // tile))
+    # (-1: the SpMV has tiles of these items too, 480 untuned, and may have built them)
+    assert tiles == -(-(A.nrow + A.nnz) // tile) or (tiles == -1 and tile in (224, 352, 480))
     yo, ya = O.spmm(A.row_ptr, A.col, stored_values(A, dtype), X, k=k)
     for _ in range(3):  # both parities
         Y = plan.spmm(Xd, alpha=-0.5, beta=0.0)
