@@ -144,10 +144,8 @@ SpmmShape spmm_shape(const merbit_plan_s* p, int cols, const SpmmOperands& o) {
     // against 64 at 256), in FP64 of 224-item ones (73 us against 84 at 352 and 82 at
     // 256; Zipf-1M 208 against 264 and 260; a 400 x 400 5-point grid 16.5 against 19
     // and 17).  One column takes 480 items, unless 256-item tiles fill one round at
-    // most: FP32 R-MAT-300k 45 us against 53 at 256, an 80 x 70 x 60 27-point stencil 45
-    // against 56, the 5-point grid 10.2 against 12.8; R-MAT-20k 13.8 against 11.9.  With
-    // the fused dval 480 in FP64 from three rounds on (Zipf-300k 88 us against 98;
-    // R-MAT-20k, half a round, 17.9 against 18.4); not in FP32 (R-MAT-300k 98 against 91).
+    // most: FP32 R-MAT-300k 47 us against 52 at 256, an 80 x 70 x 60 27-point stencil 44
+    // against 54, the 5-point grid 9.7 against 13.7; R-MAT-20k 14.3 against 11.8.
     // Other shapes keep 256.
     int items = kDefaultItems;
     const bool dv = o.dv_out != nullptr;
@@ -155,10 +153,8 @@ SpmmShape spmm_shape(const merbit_plan_s* p, int cols, const SpmmOperands& o) {
         items = spmm_odd_tile(kk);
     } else if (kk == 2 && !dv && width(352) == 2) {
         items = p->dtype == MERBIT_F64 ? 224 : 352;
-    } else if (kk == 1) {
-        const bool long_enough = dv ? p->dtype == MERBIT_F64 && tile_rounds(p, 1, 1, 480, true) >= 3
-                                    : tile_rounds(p, 1, 1, 256, false) > 1;
-        if (long_enough) items = 480;
+    } else if (kk == 1 && !dv && tile_rounds(p, 1, 1, 256, false) > 1) {
+        items = 480;
     }
     int vw = width(items);
     // Vector width 2 in tiles of an odd length per lane group: where the operands

@@ -963,8 +963,15 @@ struct SpmmStage {
 // fused dval, with two tile sizes or with 8 scalar gathers ahead would spill
 // at 5; FP32 with staged products takes 6 (80 registers; an 80 x 70 x 60
 // 27-point stencil at k = 2: 80, 71, 68 and 76 us at 4, 5, 6 and 7).
+//
+// One column, one lane per group, is the most latency-bound: FP32 takes 6, with the
+// fused dval 7 (72 registers), FP64 5 (us at 5, 6, 7 and 8: Zipf-1M FP32 product in
+// 480-item tiles 145, 144, 145, 204 and random rows of 0 to 40 29, 24, 27, 42; backward in
+// 256-item tiles Zipf-1M 270, 250, 251, 238, the stencil 83, 76, 72, 68, R-MAT-300k 84, 84,
+// 87, 88; FP64 backward at 4, 5, 6 R-MAT-300k 99, 94, 100, Zipf-300k 96, 89, 89).
 constexpr int spmm_ctas(int dt, int k, int vw, int items, int items2, bool dv) {
-    if (dt == MERBIT_F64) return dv || items2 != 0 || (vw == 1 && k > 1) ? 4 : 5;
+    if (k == 1) return dt == MERBIT_F64 ? 5 : dv ? 7 : 6;
+    if (dt == MERBIT_F64) return dv || items2 != 0 || vw == 1 ? 4 : 5;
     return spmm_staged_products(k, vw, items, dv) ? 6 : 5;
 }
 

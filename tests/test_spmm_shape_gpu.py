@@ -68,7 +68,7 @@ def _ends_at(tile, seg, items, seed):
 def test_one_and_two_columns_at_tile_ends(dtype, k, tile):
     tile = tile or (224 if dtype == "f64" else 352)
     few = tile == 256  # one round of 256-item tiles
-    A = _ends_at(tile, tile // 32, 400_000 if few else 256 * _warps(5) + 50_000, seed=k)
+    A = _ends_at(tile, tile // 32, 400_000 if few else 256 * _warps(6) + 50_000, seed=k)
     xy = np.float64 if dtype == "f64" else np.float32
     X = synth.uniform(7, A.ncol * k).reshape(A.ncol, k).astype(xy)
     plan = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
@@ -86,8 +86,8 @@ def test_one_and_two_columns_at_tile_ends(dtype, k, tile):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["f64", "f32"])
 def test_one_column_fused_backward_at_tile_ends(dtype):
-    """Three rounds of 480-item tiles (FP64) on the transpose plan."""
-    B = _ends_at(480, 15, 2 * 480 * _warps(5) + 50_000, seed=3)
+    """More than one round of 256-item tiles on the transpose plan."""
+    B = _ends_at(256, 8, 256 * _warps(7) + 50_000, seed=3)
     rows = np.repeat(np.arange(B.nrow, dtype=np.int32), np.diff(B.row_ptr))
     order = np.lexsort((rows, B.col))
     rp = np.concatenate([[0], np.cumsum(np.bincount(B.col, minlength=B.ncol))]).astype(np.int32)
