@@ -26,9 +26,9 @@
 // without passing through double when alpha = 1 and beta = 0, and only the
 // slots that a launch uses are emptied for the next one (all of them, they
 // were 20 MB of L2 for Zipf-1M at k = 16, whose X of 64 MB then no longer fit).
-// Measured on B200 (one launch of a CUDA graph): Zipf-1M FP32 k = 16 351 us, its
-// fused backward 537; Zipf-500k FP64 k = 8 153; 32 R-MAT matrices FP32 in one
-// launch, k = 4 435 us, k = 32 1,070.
+// Measured on B200 (one launch of a CUDA graph): Zipf-1M FP32 k = 16 347 us, its
+// fused backward 525; Zipf-500k FP64 k = 8 147; 32 R-MAT matrices FP32 in one
+// launch, k = 4 431 us, k = 32 1,090.
 //
 // Batches: the tiles of all matrices form one index space; matrix m owns
 // tiles [tile_begin_m, tile_begin_m + num_tiles_m).  Warps of the
