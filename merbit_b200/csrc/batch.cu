@@ -254,7 +254,10 @@ int spmm_reserve(merbit_plan_s* p, const SpmmShape& h, cudaStream_t s, bool* roo
         st = alloc_spmm_slots(&sl, (long long)part->num_tiles * h.kk, s);
         if (st == MERBIT_OK) p->spmm_slots.emplace(slot_key(h), sl);
     }
-    if (st != MERBIT_OK) *room = !out_of_memory();
+    if (st != MERBIT_OK) {
+        *room = !out_of_memory();
+        cudaStreamSynchronize(s);  // the partition stays with the plan
+    }
     return st;
 }
 
@@ -367,6 +370,12 @@ int batch_vw(const merbit_batch_s* b, int items) {
     return spmm_config_exists(b->k, vw, items) ? vw : 1;
 }
 
+// A failure after partitions were queued on s, which stay with their plans.
+int synchronized(int st, cudaStream_t s) {
+    cudaStreamSynchronize(s);
+    return st;
+}
+
 // The SpMM kernel, matrix i with tiles of tile[i] merge items (each `items`
 // or `items2`; items2 = 0: `items` for every matrix).
 int batch_build_tiles(merbit_batch_s* b, int items, int items2, const std::vector<int>& tile,
@@ -383,14 +392,15 @@ int batch_build_tiles(merbit_batch_s* b, int items, int items2, const std::vecto
         const int ti = items2 && tile[i] == items2 ? items2 : items;
         const Partition* part = nullptr;
         int st = plan_partition(b->plans[i], ti, &part, s);
-        if (st != MERBIT_OK) return st;
-        if (tot + part->num_tiles > INT_MAX) return fail(MERBIT_ERR_OVERFLOW, "batch: too many tiles");
+        if (st == MERBIT_OK && tot + part->num_tiles > INT_MAX)
+            st = fail(MERBIT_ERR_OVERFLOW, "batch: too many tiles");
+        if (st != MERBIT_OK) return synchronized(st, s);
         h[i] = make_desc(b->plans[i], part, b->x[i], b->ldx[i], b->y[i], b->ldy[i], (int)tot);
         h[i].ipt = ti;
         tot += part->num_tiles;
     }
     int st = batch_upload(b, h, tot, s);
-    if (st != MERBIT_OK) return st;
+    if (st != MERBIT_OK) return synchronized(st, s);
     b->kernel = 0;
     b->items = items;
     b->items2 = items2;
@@ -434,14 +444,15 @@ int batch_build_warp(merbit_batch_s* b, int variant, cudaStream_t s) {
         b->ipt[i] = ipt_for_variant(variant, b->ipt[i]);
         const Partition* part = nullptr;
         int st = plan_partition(b->plans[i], 32 * b->ipt[i], &part, s);
-        if (st != MERBIT_OK) return st;
-        if (tot + part->num_tiles > INT_MAX) return fail(MERBIT_ERR_OVERFLOW, "batch: too many tiles");
+        if (st == MERBIT_OK && tot + part->num_tiles > INT_MAX)
+            st = fail(MERBIT_ERR_OVERFLOW, "batch: too many tiles");
+        if (st != MERBIT_OK) return synchronized(st, s);
         h[i] = make_desc(b->plans[i], part, b->x[i], b->ldx[i], b->y[i], b->ldy[i], (int)tot);
         h[i].ipt = b->ipt[i];
         tot += part->num_tiles;
     }
     int st = batch_upload(b, h, tot, s);
-    if (st != MERBIT_OK) return st;
+    if (st != MERBIT_OK) return synchronized(st, s);
     b->kernel = 1;
     b->variant = variant;
     b->items = 0;

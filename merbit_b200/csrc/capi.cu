@@ -73,13 +73,16 @@ int grow_carry(merbit_plan_s* p, int tiles, cudaStream_t s) {
     return MERBIT_OK;
 }
 
-// Starts a partition for `tile_items` without synchronizing; its largest
-// rows-per-tile lands in p->scratch->max_rows for the caller's next
-// readback.  On failure nothing is added to the plan.
-int plan_partition_start(merbit_plan_s* p, int tile_items, Partition** out, cudaStream_t s) {
+}  // namespace
+
+int plan_partition(merbit_plan_s* p, int tile_items, const Partition** out, cudaStream_t s) {
+    for (auto& q : p->parts)
+        if (q.tile_items == tile_items) {
+            *out = &q;
+            return MERBIT_OK;
+        }
     Partition q;
-    int st = build_partition_async(p->row_ptr, p->nrow, p->nnz, tile_items, &q,
-                                   &p->scratch->max_rows, s);
+    const int st = build_partition_async(p->row_ptr, p->nrow, p->nnz, tile_items, &q, s);
     if (st != MERBIT_OK) {
         dev_free(q.coords, s);
         return st;
@@ -89,42 +92,36 @@ int plan_partition_start(merbit_plan_s* p, int tile_items, Partition** out, cuda
     return MERBIT_OK;
 }
 
-}  // namespace
-
-int plan_partition(merbit_plan_s* p, int tile_items, const Partition** out, cudaStream_t s) {
-    for (auto& q : p->parts)
-        if (q.tile_items == tile_items) {
-            *out = &q;
-            return MERBIT_OK;
-        }
-    Partition* q = nullptr;
-    int st = plan_partition_start(p, tile_items, &q, s);
-    if (st != MERBIT_OK) return st;
-    int h_max = 0;
-    cudaError_t e = cudaMemcpyAsync(&h_max, &p->scratch->max_rows, sizeof(int),
-                                    cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        dev_free(q->coords, s);
-        p->parts.pop_back();
-        return cuda_fail(e, "partition: max rows");
-    }
-    q->max_rows = h_max;
-    *out = q;
-    return MERBIT_OK;
-}
-
 namespace {
 
-// The partition of an SpMV configuration, with carry words for its tiles.
-// (SpMM and batch launches bring words of their own, SpmmSlots, and take the
-// partition alone.)
+// The partition of an SpMV configuration, with its largest rows-per-tile and
+// carry words for its tiles.  (SpMM and batch launches take any rows per tile and
+// bring words of their own, SpmmSlots: they need the coordinates alone.)
 int spmv_partition(merbit_plan_s* p, int tile_items, const Partition** out, cudaStream_t s) {
     int st = plan_partition(p, tile_items, out, s);
-    if (st != MERBIT_OK || (*out)->num_tiles <= p->carry.slots) return st;
-    st = grow_carry(p, (*out)->num_tiles, s);
     if (st != MERBIT_OK) return st;
-    MERBIT_CUDA(cudaStreamSynchronize(s));
+    const bool rows = (*out)->max_rows < 0, words = (*out)->num_tiles > p->carry.slots;
+    if (!rows && !words) return MERBIT_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    MERBIT_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone)  // before anything is queued
+        return fail(MERBIT_ERR_INVALID,
+                    "the stream is being captured and the plan has not run this configuration: "
+                    "select it (or make its first product) before capture");
+    int h_max = (*out)->max_rows;
+    if (words) st = grow_carry(p, (*out)->num_tiles, s);
+    if (st == MERBIT_OK && rows) {
+        st = max_rows_async(**out, &p->scratch->max_rows, s);
+        if (st == MERBIT_OK) {
+            const cudaError_t e = cudaMemcpyAsync(&h_max, &p->scratch->max_rows, sizeof(int),
+                                                  cudaMemcpyDeviceToHost, s);
+            if (e != cudaSuccess) st = cuda_fail(e, "partition: max rows");
+        }
+    }
+    const cudaError_t e = cudaStreamSynchronize(s);  // the partition, whatever failed
+    if (st != MERBIT_OK) return st;
+    if (e != cudaSuccess) return cuda_fail(e, "partition");
+    const_cast<Partition*>(*out)->max_rows = h_max;
     return MERBIT_OK;
 }
 
@@ -448,10 +445,12 @@ int merbit_plan_create(merbit_plan* plan, int32_t nrow, int32_t ncol, int32_t nn
         first = provisional;
     for (int i = 0, n = spmv_num_configs(dtype); first < 0 && i < n; ++i)
         if (spmv_config_allowed(spmv_config(dtype, i), p->vec)) first = i;
-    Partition* part = nullptr;
-    if (st == MERBIT_OK && first >= 0 && spmv_config(dtype, first).kind != 3)
-        st = plan_partition_start(p, spmv_tile_items(spmv_config(dtype, first)), &part, s);
-    if (st == MERBIT_OK && part) st = grow_carry(p, part->num_tiles, s);
+    const Partition* part = nullptr;
+    if (st == MERBIT_OK && first >= 0 && spmv_config(dtype, first).kind != 3) {
+        st = plan_partition(p, spmv_tile_items(spmv_config(dtype, first)), &part, s);
+        if (st == MERBIT_OK) st = max_rows_async(*part, &p->scratch->max_rows, s);
+        if (st == MERBIT_OK) st = grow_carry(p, part->num_tiles, s);
+    }
     PlanScratch h = {};
     if (st == MERBIT_OK) {
         e = cudaMemcpyAsync(&h, p->scratch, sizeof(h), cudaMemcpyDeviceToHost, s);
@@ -461,7 +460,7 @@ int merbit_plan_create(merbit_plan* plan, int32_t nrow, int32_t ncol, int32_t nn
     if (st == MERBIT_OK && validate) st = validate_status(h);
     if (st == MERBIT_OK) {
         p->max_row_len = h.max_row_len;
-        if (part) part->max_rows = h.max_rows;
+        if (part) const_cast<Partition*>(part)->max_rows = h.max_rows;
         // the exact signature, longest row included
         int tuned = -1;
         {

@@ -380,7 +380,7 @@ inline size_t xy_size(int dt) { return dt == MERBIT_F64 ? 8 : 4; }
 struct Partition {
     int tile_items = 0;
     int num_tiles = 0;
-    int max_rows = 0;  // largest number of row ends in one tile
+    int max_rows = 0;  // largest number of row ends in one tile (-1: not known)
     int2* coords = nullptr;
 };
 
@@ -390,10 +390,12 @@ struct Partition {
 constexpr int warp_rp_cap(int ipt) { return (32 * ipt) / 3 + 16; }
 
 // Allocates out->coords and queues the merge-path search of every tile
-// boundary on s, without synchronizing; the largest rows-per-tile lands in
-// *d_max_rows, and out->max_rows stays -1 until the caller reads it back.
+// boundary on s, without synchronizing; out->max_rows is -1 until an SpMV
+// configuration needs it.
 int build_partition_async(const int32_t* row_ptr, int nrow, int nnz, int tile_items,
-                          Partition* out, int* d_max_rows, cudaStream_t s);
+                          Partition* out, cudaStream_t s);
+// Queues the partition's largest rows-per-tile into *d_max_rows.
+int max_rows_async(const Partition& part, int* d_max_rows, cudaStream_t s);
 
 // Device words a plan build reads back once: validation result (error bits,
 // first decreasing row, first bad column) and the new partition's largest
@@ -709,7 +711,8 @@ struct merbit_plan_s {
 };
 
 namespace merbit {
-// The plan's partition for `tile_items` (coordinates alone; built, with one
-// synchronization of s, when the plan has none).
+// The plan's partition for `tile_items`: coordinates alone, queued on s when the
+// plan has none.  Callers synchronize s before a launch on another stream can use
+// it.
 int plan_partition(merbit_plan_s* p, int tile_items, const Partition** out, cudaStream_t s);
 }

@@ -146,7 +146,7 @@ __global__ void max_rows_kernel(const int2* __restrict__ coords, int num_tiles,
 }
 
 int build_partition_async(const int32_t* row_ptr, int nrow, int nnz, int tile_items,
-                          Partition* out, int* d_max_rows, cudaStream_t s) {
+                          Partition* out, cudaStream_t s) {
     const long long total = (long long)nrow + nnz;
     const long long T = (total + tile_items - 1) / tile_items;
     if (T > INT_MAX - 2) return fail(MERBIT_ERR_OVERFLOW, "partition: too many tiles");
@@ -156,17 +156,21 @@ int build_partition_async(const int32_t* row_ptr, int nrow, int nnz, int tile_it
     // before anything is queued: it is refused while s is being captured
     int st = dev_alloc(&out->coords, sizeof(int2) * (size_t)(T + 1), s);
     if (st != MERBIT_OK) return st;
-    MERBIT_CUDA(cudaMemsetAsync(d_max_rows, 0, sizeof(int), s));
     const long long count = T + 1;
     const int bs = 256;
     const unsigned grid = (unsigned)((count + bs - 1) / bs);
     merge_coords_kernel<<<grid, bs, 0, s>>>(row_ptr, nrow, nnz, tile_items, count, nullptr,
                                             nullptr, out->coords);
     MERBIT_CUDA(cudaGetLastError());
-    // largest rows-per-tile, which decides the configurations the plan can use
+    return MERBIT_OK;
+}
+
+int max_rows_async(const Partition& part, int* d_max_rows, cudaStream_t s) {
+    MERBIT_CUDA(cudaMemsetAsync(d_max_rows, 0, sizeof(int), s));
+    const long long T = part.num_tiles;
     if (T > 0) {
-        max_rows_kernel<<<(unsigned)min((T + 255) / 256, 1024LL), 256, 0, s>>>(out->coords, (int)T,
-                                                                               d_max_rows);
+        max_rows_kernel<<<(unsigned)min((T + 255) / 256, 1024LL), 256, 0, s>>>(
+            part.coords, part.num_tiles, d_max_rows);
         MERBIT_CUDA(cudaGetLastError());
     }
     return MERBIT_OK;

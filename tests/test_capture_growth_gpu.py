@@ -132,3 +132,37 @@ def test_captured_residual_after_more_partials():
     g.replay()
     torch.cuda.synchronize()
     assert float(res) == ref and torch.equal(y, yref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_partitions_of_other_launches_are_checked_for_the_spmv(dtype):
+    """A batch and an SpMM leave coordinates alone; an SpMV configuration on the
+    same tiles still finds out whether its row_ptr window holds them."""
+    L = [300] + [0] * 4000 + [1, 0] * 900 + [2000] + [40] * 700
+    rp = np.concatenate([[0], np.cumsum(L)]).astype(np.int32)
+    rng = np.random.default_rng(3)
+    nnz = int(rp[-1])
+    A = synth.CSR(rp, rng.integers(0, 3000, nnz, dtype=np.int32), rng.standard_normal(nnz), 3000, "runs")
+    xy = np.float64 if dtype == "f64" else np.float32
+    xh = synth.uniform(4, A.ncol).astype(xy)
+    yo, ya = O.spmm(A.row_ptr, A.col, stored_values(A, dtype), xh)
+    x = torch.from_numpy(xh).cuda()
+    fresh = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
+    plan = mb.Plan(*to_cuda(A, dtype), ncol=A.ncol)
+    y = torch.empty(A.nrow, 1, dtype=x.dtype, device="cuda")
+    b = mb.Batch([plan], [x.view(-1, 1)], [y])
+    for variant, ipts in ((0, (7, 11, 15)), (3, (15, 19, 23))):
+        b.set_kernel(1, variant)
+        for ipt in ipts:
+            b.set_matrix_config(0, ipt)
+    b.run()
+    plan.spmm(x.view(-1, 1).expand(-1, 2).contiguous())
+    usable = plan.configs()
+    assert usable == fresh.configs()
+    assert len(usable) < mb.lib().merbit_num_configs(plan.dtype)
+    for idx, *_ in usable:
+        plan.set_config(idx)
+        got = plan.spmv(x).cpu().numpy()
+        assert (np.abs(got - yo) <= TOL[dtype] * np.maximum(ya, 1e-300)).all(), idx
+    plan.check()
