@@ -968,9 +968,13 @@ struct SpmmStage {
 // fused dval 7 (72 registers), FP64 5 (us at 5, 6, 7 and 8: Zipf-1M FP32 product in
 // 480-item tiles 145, 144, 145, 204 and random rows of 0 to 40 29, 24, 27, 42; backward in
 // 256-item tiles Zipf-1M 270, 250, 251, 238, the stencil 83, 76, 72, 68, R-MAT-300k 84, 84,
-// 87, 88; FP64 backward at 4, 5, 6 R-MAT-300k 99, 94, 100, Zipf-300k 96, 89, 89).
+// 87, 88; FP64 backward at 4, 5, 6 R-MAT-300k 99, 94, 100, Zipf-300k 96, 89, 89).  The
+// FP32 backward of two columns takes 7 as well (at 5, 6 and 7 the stencil 95, 94, 88,
+// the random rows 50, 46, 43, R-MAT-40k 22, 25, 20, Zipf-1M 285, 275, 287, R-MAT-300k 93,
+// 97, 102).
 constexpr int spmm_ctas(int dt, int k, int vw, int items, int items2, bool dv) {
     if (k == 1) return dt == MERBIT_F64 ? 5 : dv ? 7 : 6;
+    if (k == 2 && vw == 2 && dv && dt != MERBIT_F64) return 7;
     if (dt == MERBIT_F64) return dv || items2 != 0 || vw == 1 ? 4 : 5;
     return spmm_staged_products(k, vw, items, dv) ? 6 : 5;
 }
