@@ -164,9 +164,11 @@ int merbit_spmv(merbit_plan plan, double alpha, const void* d_x, double beta, vo
  *     y = damp * A x + (1 - damp) * teleport
  *     *d_residual = sum_i |y_i - x_i|   (L1, of y as stored; skipped if NULL)
  * The residual is reduced inside the SpMV launch -- per-CTA partials summed in
- * a fixed order by the launch's last CTA -- so it is deterministic and costs
- * no extra pass over y.  The plan must be square; x, teleport and y are
- * vectors of the plan's x/y type; y must not alias x (teleport may alias y).
+ * a fixed order by the launch's last CTA -- and costs no extra pass over y.  y
+ * repeats bit for bit; the residual does up to its last bits (with warp tiles the
+ * term of a row that two tiles share is added by the tile that finishes it, either
+ * one).  The plan must be square; x, teleport and y are vectors of the plan's x/y
+ * type; y must not alias x (teleport may alias y).
  * A row without nonzeros gets only the teleport term; the rank of a node
  * without out-links is not redistributed (plain power step). */
 int merbit_pagerank_step(merbit_plan plan, double damp, const void* d_x, const void* d_teleport,

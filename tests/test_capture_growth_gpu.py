@@ -104,10 +104,12 @@ def test_captured_spmv_after_a_configuration_of_more_tiles(eager):
 
 @pytest.mark.gpu
 def test_captured_residual_after_more_partials():
-    """More CTAs than the captured step had: its partial sums keep their place."""
+    """More CTAs than the captured step had: its partial sums keep their place.  On
+    CTA tiles, where one tile finishes each row and the residual repeats bit for bit
+    (warp tiles that share a row leave its term to the later one)."""
     A = synth.laplace2d(1100, 1000)
     plan = mb.Plan(*to_cuda(A, "f64"), ncol=A.ncol)
-    plan.set_config(0)
+    plan.set_config(next(c for c in plan.configs() if c[1] == 0 and c[2] * c[3] == 1792)[0])
     n = A.nrow
     x = torch.from_numpy(synth.uniform(2, n)).cuda()
     t = torch.full((n,), 1.0 / n, dtype=torch.float64, device="cuda")
